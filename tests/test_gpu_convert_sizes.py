@@ -1,0 +1,77 @@
+"""GPU parity of the conversion where its kernels change method: blocks of exactly / one more than the entries a warp or a
+CTA sorts, lists longer than one slice of columns, more columns than one bitmap pass holds, repeated entries in short and
+long panels, a short last panel.  Bit-exact against the CPU checker, so there is no tolerance."""
+import numpy as np
+import pytest
+
+import _orc
+
+pytestmark = pytest.mark.gpu
+
+SIZES = (0, 1, 127, 128, 129, 256, 257, 512, 513, 1024, 1025, 4096, 4097, 9000, 30000)
+
+
+def blocks_csr(sizes, cols, last_rows, repeats, seed):
+    """One 8-row block per size (the last of `last_rows` rows), entries spread unevenly over its rows, unsorted; `repeats`
+    duplicates a few (row, col) pairs of every block."""
+    rng = np.random.Generator(np.random.Philox(seed))
+    lens, ci = [], []
+    for i, n in enumerate(sizes):
+        rows = 8 if i + 1 < len(sizes) else last_rows
+        split = np.bincount(np.minimum(rng.geometric(0.4, size=n) - 1, rows - 1), minlength=rows)
+        split = np.minimum(split, cols)
+        shared = rng.choice(cols, size=min(cols, 64), replace=False)
+        for k in split:
+            c = rng.choice(cols, size=int(k), replace=False)
+            c[: k // 3] = rng.permutation(np.unique(np.concatenate([c[: k // 3], shared])))[: k // 3]
+            if repeats and k > 2:
+                c[-1] = c[0]
+            lens.append(int(k))
+            ci.append(c.astype(np.int32))
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    ci = np.concatenate(ci).astype(np.int32)
+    return rp, ci, rng.uniform(-1.0, 1.0, size=ci.size).astype(np.float32), (rp.size - 1, cols)
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("cols,repeats", [(40000, False), (40000, True), ((1 << 20) + 5, False), (300, True)])
+def test_conversion_at_the_edges_of_its_methods(prec, cols, repeats):
+    from tilespmm_b200 import api
+    m = api.TileMatrix(prec)
+    for seed, last_rows in ((1, 8), (2, 3)):
+        order = np.random.default_rng(seed).permutation(SIZES)
+        rp, ci, v, shape = blocks_csr(order.tolist(), cols, last_rows, repeats, seed)
+        vv = api.to_values(v, prec)
+        for g, d in ((5.0, 3.0), (5.0, 0.0), (0.0, 1.5), (2.0, 1.2), (4.0, 1.4)):
+            m.convert_host(shape, rp, ci, vv, g, d)
+            o = _orc.Orc(prec, shape, rp, ci, vv, g, d)
+            assert m.info().tolist() == o.info().tolist(), (g, d)
+            for cls in range(3):
+                for w in _orc.ARRAYS:
+                    np.testing.assert_array_equal(m.array(cls, w), o.array(cls, w), err_msg=f"{g},{d} class {cls} {w}")
+    m.close()
+
+
+@pytest.mark.parametrize("tasks", [2047, 2048, 2049, 70000])
+def test_schedule_at_the_edge_of_the_one_block_builder(tasks):
+    """Up to 2048 panels and tasks one CTA builds the schedule; the task list and the walked copy must cover the same tiles."""
+    import torch
+    from tilespmm_b200 import api
+    rp = (np.arange(8 * tasks + 1) // 8).astype(np.int32)              # one entry per panel ...
+    rp[8:] += 40
+    rp[1:8] += np.linspace(5, 40, 7).astype(np.int32)                  # ... and a longer first panel, which TH = 1 splits
+    nnz = int(rp[-1])
+    ci = (np.arange(nnz) * 7 % 4001).astype(np.int32)
+    shape = (8 * tasks, 4001)
+    m = api.TileMatrix(0).convert_host(shape, rp, ci, np.ones(nnz, np.float32), 5.0, 3.0)
+    o = _orc.Orc(0, shape, rp, ci, api.to_values(np.ones(nnz, np.float32), 0), 5.0, 3.0)
+    assert m.info().tolist() == o.info().tolist()
+    B = torch.ones((shape[1], 32), dtype=torch.float16, device="cuda")
+    C = torch.full((m.c_rows(), 32), 7.0, dtype=torch.float32, device="cuda")
+    for TH in (1, 8):
+        rows, start = m.schedule(2, TH)
+        assert start[0] == 0 and start[-1] == int(m.info()[2, 3]) and (np.diff(start) <= TH).all()
+        m.spmm(B, C, 32)
+        torch.cuda.synchronize()
+        np.testing.assert_array_equal(C[: shape[0], 0].cpu().numpy(), np.diff(rp).astype(np.float32))
+    m.close()

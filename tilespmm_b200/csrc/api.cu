@@ -83,6 +83,7 @@ static int create_resources(tsp_handle *h)
         TSP_CUDA(cudaEventCreateWithFlags(&h->join[i], cudaEventDisableTiming));
     }
     TSP_CUDA(cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming));
+    TSP_CUDA(cudaEventCreateWithFlags(&h->sched_ready, cudaEventDisableTiming));
     TSP_CUDA(cudaEventCreate(&h->t0));
     TSP_CUDA(cudaEventCreate(&h->t1));
     TSP_CUDA(cudaMalloc((void **)&h->d_error, 4));
@@ -99,6 +100,8 @@ extern "C" int tsp_destroy(tsp_handle *h)
     tsp_free_workspace(h);
     if (h->h_pin) cudaFreeHost(h->h_pin);
     for (int i = 0; i < 2; i++) { if (h->side[i]) cudaStreamDestroy(h->side[i]); if (h->join[i]) cudaEventDestroy(h->join[i]); }
+    cudaFree(h->sched_scratch);
+    if (h->sched_ready) cudaEventDestroy(h->sched_ready);
     if (h->fork) cudaEventDestroy(h->fork);
     if (h->t0) cudaEventDestroy(h->t0);
     if (h->t1) cudaEventDestroy(h->t1);
@@ -152,6 +155,7 @@ extern "C" int tsp_export(const tsp_handle *h, int cls, int which, void *dst, lo
     const size_t vsz = h->precision ? 4 : 2;
     *bytes = 0;
     if (c.rows == 0 && which != 7) return TSP_OK;
+    if (dst && (which == 0 || which == 1 || which == 5)) TSP_TRY(tsp_fetch_panels(h, cls));
     switch (which)
     {
     case 0:  // orig_row: the rows of every panel, in panel order (src/hetero_split.h:86-141)
@@ -232,8 +236,42 @@ static int check_width(int colB)
     return TSP_EINVAL;
 }
 
-static int ensure_schedules(tsp_handle *h, int colB)
+// restores the calling thread's stream-capture mode
+struct RelaxedCapture
 {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// Schedules of the first candidate threshold for the classes that have none yet, enqueued on `s`.  A later call on another
+// stream must not overtake them: it waits for their event -- on the host, once, because a stream that is being captured
+// may neither wait for an event from outside the capture nor query it.  A call that is itself being captured builds them
+// outside the capture and waits.
+static int ensure_schedules(tsp_handle *h, int colB, cudaStream_t s)
+{
+    bool built = false;
+    const cudaStream_t caller = s;
+    for (int k = 0; k < 3 && !built; k++) built = h->cls[k].tilem > 0 && h->cls[k].TH == 0;
+    if (built)
+    {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) { cudaGetLastError(); cs = cudaStreamCaptureStatusNone; }
+        if (cs != cudaStreamCaptureStatusNone) s = h->side[0];
+    }
+    if (s != caller)
+    {
+        RelaxedCapture relaxed;
+        for (int k = 0; k < 3; k++)
+            if (h->cls[k].tilem > 0 && h->cls[k].TH == 0)
+            {
+                int top4[4];
+                TSP_TRY(tsp_top4(h, k, colB, top4));
+                TSP_TRY(tsp_schedule_on(h, k, top4[0], s));
+            }
+        TSP_CUDA(cudaStreamSynchronize(s));
+        return TSP_OK;
+    }
     for (int k = 0; k < 3; k++)
     {
         TspClass &c = h->cls[k];
@@ -241,8 +279,19 @@ static int ensure_schedules(tsp_handle *h, int colB)
         {
             int top4[4];
             TSP_TRY(tsp_top4(h, k, colB, top4));
-            TSP_TRY(tsp_schedule(h, k, top4[0]));
+            TSP_TRY(tsp_schedule_on(h, k, top4[0], s));
         }
+    }
+    if (built)
+    {
+        TSP_CUDA(cudaEventRecord(h->sched_ready, s));
+        h->sched_stream = s; h->sched_pending = true;
+    }
+    else if (h->sched_pending && s != h->sched_stream)
+    {
+        RelaxedCapture relaxed;
+        TSP_CUDA(cudaEventSynchronize(h->sched_ready));
+        h->sched_pending = false;
     }
     return TSP_OK;
 }
@@ -354,7 +403,7 @@ extern "C" int tsp_spmm(tsp_handle *h, const void *d_b, float *d_c, int colB, vo
     if (!h->converted) { tsp_set_error("spmm: convert first"); return TSP_ESTATE; }
     TSP_TRY(check_width(colB));
     TSP_CUDA(cudaSetDevice(h->device));
-    TSP_TRY(ensure_schedules(h, colB));
+    TSP_TRY(ensure_schedules(h, colB, (cudaStream_t)stream));
     return spmm_on(h, d_b, d_c, colB, (cudaStream_t)stream);
 }
 
@@ -402,7 +451,7 @@ extern "C" int tsp_spmm_host_async(tsp_handle *h, const void *h_b, float *h_c, i
     const size_t vsz = h->precision ? 4 : 2;
     const size_t b_bytes = (size_t)h->colA * colB * vsz, c_bytes = (size_t)tsp_c_rows(h) * colB * 4;
     TSP_TRY(ensure_staging(h, slot, b_bytes, c_bytes));
-    TSP_TRY(ensure_schedules(h, colB));
+    TSP_TRY(ensure_schedules(h, colB, h->s_cmp));
     TSP_CUDA(cudaMemcpyAsync(h->stage_b[slot], h_b, b_bytes, cudaMemcpyHostToDevice, h->s_in));
     TSP_CUDA(cudaEventRecord(h->ev_in[slot], h->s_in));
     TSP_CUDA(cudaStreamWaitEvent(h->s_cmp, h->ev_in[slot], 0));
@@ -469,8 +518,8 @@ extern "C" int tsp_time(tsp_handle *h, int cls, const void *d_b, float *d_c, int
     if (!h->converted) { tsp_set_error("time: convert first"); return TSP_ESTATE; }
     TSP_TRY(check_width(colB));
     TSP_CUDA(cudaSetDevice(h->device));
-    TSP_TRY(ensure_schedules(h, colB));
     cudaStream_t s = 0;
+    TSP_TRY(ensure_schedules(h, colB, s));
     TSP_CUDA(cudaEventRecord(h->t0, s));
     for (int i = 0; i < iters; i++)
     {
@@ -506,7 +555,7 @@ extern "C" int tsp_tune(tsp_handle *h, const void *d_b, float *d_c, int colB, in
             if (!dup) cand[k][ncand[k]++] = top4[i];
         }
         best3[k] = cand[k][0];
-        if (h->cls[k].tilem > 0) TSP_TRY(tsp_schedule(h, k, cand[k][0]));
+        if (h->cls[k].tilem > 0) TSP_TRY(tsp_schedule_on(h, k, cand[k][0], 0));
     }
     cudaStream_t s = 0;
     cudaEvent_t a, b;
@@ -522,7 +571,7 @@ extern "C" int tsp_tune(tsp_handle *h, const void *d_b, float *d_c, int colB, in
                 {
                     const int th[3] = {cand[0][i], cand[1][j], cand[2][k]};
                     for (int q = 0; q < 3; q++)
-                        if (h->cls[q].tilem > 0 && h->cls[q].TH != th[q]) TSP_TRY(tsp_schedule(h, q, th[q]));
+                        if (h->cls[q].tilem > 0 && h->cls[q].TH != th[q]) TSP_TRY(tsp_schedule_on(h, q, th[q], s));
                     for (int w = 0; w < 5; w++) TSP_TRY(spmm_on(h, d_b, d_c, colB, s));
                     TSP_CUDA(cudaEventRecord(h->t0, s));
                     for (int w = 0; w < 10; w++) TSP_TRY(spmm_on(h, d_b, d_c, colB, s));
@@ -533,7 +582,7 @@ extern "C" int tsp_tune(tsp_handle *h, const void *d_b, float *d_c, int colB, in
                     if (ms < best_ms) { best_ms = ms; best3[0] = th[0]; best3[1] = th[1]; best3[2] = th[2]; }
                 }
         for (int q = 0; q < 3; q++)
-            if (h->cls[q].tilem > 0 && h->cls[q].TH != best3[q]) TSP_TRY(tsp_schedule(h, q, best3[q]));
+            if (h->cls[q].tilem > 0 && h->cls[q].TH != best3[q]) TSP_TRY(tsp_schedule_on(h, q, best3[q], s));
     }
     TSP_CUDA(cudaEventRecord(b, s));
     TSP_CUDA(cudaEventSynchronize(b));
@@ -628,7 +677,7 @@ extern "C" int tsp_run(tsp_handle *h, const void *h_b, float *h_c, int colB, int
     // threshold candidates (host cost model) + tuning, both counted as preprocessing like upstream (src/csr2tile.h:1061)
     const double t_a = now_ms();
     for (int k = 0; k < 3; k++) h->cls[k].TH = 0;
-    if ((rc = ensure_schedules(h, colB)) != TSP_OK) return bail(rc);
+    if ((rc = ensure_schedules(h, colB, 0)) != TSP_OK) return bail(rc);
     const double cand_ms = now_ms() - t_a;
     if ((rc = warmup_like_upstream(h, d_b, d_c, colB)) != TSP_OK) return bail(rc);
     int best3[3];

@@ -1,37 +1,58 @@
 // GPU partitioning and CSR -> tile conversion.
 //
 // Replaces upstream matrix_split (src/hetero_split.h:144-291) and Tile_create (src/csr2tile.h:724-795), which
-// run on the host with per-thread column flag arrays.  Here every stage is a data-parallel kernel:
+// run on the host with per-thread column flag arrays.  The entries of an 8-row block are contiguous in the CSR, so
+// everything is done block by block in registers and shared memory; there is no sort over the whole matrix:
 //
-//   1. keys (8-row block, column) for every stored entry -> radix sort -> unique: the sorted distinct
-//      columns of every 8-row block (U8 lists, contiguous, with offsets u8_ptr).
-//   2. exact distinct-column counts of every 8/16/64-row window starting at a multiple of 8 rows
-//      (|U8|, two-list and eight-list unions by binary search) -- the N8/N16/N64 of the upstream scan.
-//   3. the upstream decision (64 / 16 / 8 rows) evaluated for EVERY 8-aligned start in parallel, with the
-//      same float comparisons, then the greedy chain i <- i + step(i) resolved chunk-wise.
-//   4. keys (panel, column) -> sort -> unique: sorted distinct columns of every panel; tiles per panel,
-//      prefix sums (tile_ptr), tile_colidx with upstream's padding.
-//   5. one warp per original row: rank of every entry in its panel's column list -> tile, slot; per-tile
-//      entry counts (tile_nnz); for the 16- and 8-row classes the dense tile values, accumulated in CSR order in
-//      value type; for the 64-row class the row masks of every tile (bitmap).
-//   6. 64-row class: entries per tile from the masks -> record sizes (packed: masks + values, dense: 4 KB) ->
-//      prefix sum (record offsets) -> values placed in mask order (repeated entries summed in CSR order).
+//   1. sorted distinct columns of every 8-row block (`ucols`, block b's list starts where its entries start in the CSR,
+//      so no compaction is needed; `ulen` = its length).  A warp sorts up to 512 columns in registers, a CTA up to 4096 in
+//      shared memory; a longer block sets bits in a bitmap of up to 2^20 columns at a time and reads them back in order.
+//   2. where windows of 16 and 64 rows are compared: for every block, how many of its columns the previous 1..7 blocks do
+//      not hold (binary searches in their lists).  The distinct columns of a window are sums of eight such counts.
+//   3. the upstream decision (64 / 16 / 8 rows) for EVERY 8-aligned start, with the same float comparisons, then the
+//      greedy chain i <- i + step(i), resolved chunk-wise; the same pass carries tiles and entries per class, so the
+//      chain's last kernel writes tile_ptr and the histogram of panel lengths directly.
+//   4. ONE read-back of a few kilobytes; allocation.
+//   5. tall panels: sorted distinct columns from the lists of their blocks (the same three methods), written as
+//      tile_colidx.
+//   6. 16- and 8-row panels: a warp builds all tiles of a panel of up to 512 entries in shared memory (values, column
+//      indices, entry counts) and writes them once; a longer panel is cut into slices of 4096 columns, a CTA each.
+//   7. 64-row panels: row masks per slice in shared memory, record sizes, one prefix sum, values into the records.
+//
+// Repeated (row, col) entries are rare: steps 6 and 7 set one bit per entry, and only a panel in which a bit was already
+// set is done again by the ordered path that adds them in CSR order in value type (src/csr2tile.h:271, 283, 318).
 //
 // tile_ptr, tile_nnz, tile_colidx, panel rows and, after expansion (tsp_export), the tile values are bit-identical to
 // upstream's for the same CSR, gamma and delta; the masks are defined by the CSR alone (an explicit zero sets its bit).
-//
-// Host side: all scratch comes from a workspace kept in the handle (no cudaMalloc/cudaFree per stage), the tile
-// arrays of all classes are one allocation, and the host reads back a handful of scalars in three small copies.
 #include <cub/cub.cuh>
+#include <stddef.h>
 #include <stdlib.h>
 #include <sys/time.h>
+
+#include <mutex>
 
 #include "tsp_internal.cuh"
 
 namespace
 {
 
-constexpr int CHAIN_L = 64;   // 8-row blocks per chunk of the chain resolution
+constexpr int CHAIN_L = 64;         // 8-row blocks per chunk of the chain resolution
+constexpr int SMALL_N = 512;        // entries a warp sorts in registers / builds tiles of in shared memory
+constexpr int MID_N = 4096;         // entries a CTA of 256 threads sorts in shared memory
+constexpr int SLICE_COLS = 4096;    // distinct columns of one slice of a long panel
+constexpr int CHUNK_N = 4096;       // entries one CTA places into the records of a 64-row panel
+
+// What the host reads back in one copy, and the counters of the device-side work lists.
+struct ConvStats
+{
+    int bad;                        // the CSR is inconsistent
+    int last_cls;                   // class of the last panel (only that one can be shorter than its class's height)
+    int panels[3], tiles[3], nnz[3];
+    int n_mid[2], n_big[2];         // blocks / panels left to the CTA-level list kernels
+    int n_items[3], n_chunks;       // slices of long panels; chunks of entries of 64-row panels
+    int max_len[3];                 // longest panel in tiles
+    int hist[3][TSP_HIST_BINS];     // panels by number of tiles; the last bin stands for every longer one
+};
 
 // Bump allocator over the handle's workspace chunks.  The first conversion sizes chunk 0 from nnz and rowA; what
 // does not fit (sizes known only later) goes into further chunks, which later conversions reuse.
@@ -80,192 +101,452 @@ int reserve_workspace(tsp_handle *h, size_t bytes)
     return TSP_OK;
 }
 
+
+// ---- sorted distinct columns of a list of keys: three methods by size
+//
+// Measured on R-MAT scale 18 (7.6 M entries, 32768 blocks, 1 - 60,000 entries each): see the table of conversion times in
+// the design notes; the global radix sort these replace moved every key eight times through memory.
+
+// bitonic sort of 32*R keys in registers, element i = lane*R + r
+template <int R>
+__device__ __forceinline__ void warp_sort(unsigned (&k)[R], int lane)
+{
+#pragma unroll
+    for (int size = 2; size <= 32 * R; size <<= 1)
+    {
+#pragma unroll
+        for (int stride = size >> 1; stride > 0; stride >>= 1)
+        {
+            if (stride >= R)
+            {
+                const int m = stride / R;
+                const bool up = size >= 32 * R || (lane & (size / R)) == 0;
+                const bool low = ((lane & m) == 0) == up;
+#pragma unroll
+                for (int r = 0; r < R; r++)
+                {
+                    const unsigned o = __shfl_xor_sync(0xffffffffu, k[r], m);
+                    k[r] = low ? min(k[r], o) : max(k[r], o);
+                }
+            }
+            else
+            {
+#pragma unroll
+                for (int r = 0; r < R; r++)
+                {
+                    const int q = r ^ stride;
+                    if (q > r)
+                    {
+                        const bool up = size >= 32 * R || (size >= R ? (lane & (size / R)) == 0 : (r & size) == 0);
+                        const unsigned a = k[r], b = k[q], lo = min(a, b), hi = max(a, b);
+                        k[r] = up ? lo : hi;
+                        k[q] = up ? hi : lo;
+                    }
+                }
+            }
+        }
+    }
+}
+
+// n <= 32*R keys load(e) -> emit(position, key) for every distinct key in ascending order; returns their number
+template <int R, typename Load, typename Emit>
+__device__ __forceinline__ int warp_sort_unique(int n, int lane, Load load, Emit emit)
+{
+    unsigned k[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) k[r] = r * 32 + lane < n ? (unsigned)load(r * 32 + lane) : 0xffffffffu;
+    warp_sort<R>(k, lane);
+    const unsigned prev = __shfl_up_sync(0xffffffffu, k[R - 1], 1);
+    unsigned heads = 0;
+#pragma unroll
+    for (int r = 0; r < R; r++)
+    {
+        const unsigned p = r ? k[r ? r - 1 : 0] : prev;
+        if (k[r] != 0xffffffffu && ((r == 0 && lane == 0) || k[r] != p)) heads |= 1u << r;
+    }
+    const int cnt = __popc(heads);
+    int incl = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += y; }
+    int pos = incl - cnt;
+#pragma unroll
+    for (int r = 0; r < R; r++) if (heads >> r & 1) emit(pos++, (int)k[r]);
+    return __shfl_sync(0xffffffffu, incl, 31);
+}
+
+template <typename Load, typename Emit>
+__device__ __forceinline__ int warp_list(int n, int lane, Load load, Emit emit)
+{
+    if (n <= 128) return warp_sort_unique<4>(n, lane, load, emit);
+    if (n <= 256) return warp_sort_unique<8>(n, lane, load, emit);
+    return warp_sort_unique<16>(n, lane, load, emit);
+}
+
+template <int ITEMS>
+struct CtaSort
+{
+    using Sort = cub::BlockRadixSort<unsigned, 256, ITEMS>;
+    using Scan = cub::BlockScan<int, 256>;
+    union Temp { typename Sort::TempStorage sort; typename Scan::TempStorage scan; };
+};
+union CtaTemp { CtaSort<4>::Temp t4; CtaSort<16>::Temp t16; };
+
+// the same by a CTA of 256 threads; n <= 256*ITEMS
+template <int ITEMS, typename Load, typename Emit>
+__device__ __forceinline__ int cta_sort_unique(typename CtaSort<ITEMS>::Temp &temp, unsigned *last /* [256] */, int n, int bits, Load load, Emit emit)
+{
+    const int tid = threadIdx.x;
+    unsigned k[ITEMS];
+#pragma unroll
+    for (int r = 0; r < ITEMS; r++) k[r] = r * 256 + tid < n ? (unsigned)load(r * 256 + tid) : 0xffffffffu;
+    typename CtaSort<ITEMS>::Sort(temp.sort).Sort(k, 0, bits);
+    last[tid] = k[ITEMS - 1];
+    __syncthreads();
+    const unsigned prev = tid ? last[tid - 1] : 0u;
+    unsigned heads = 0;
+#pragma unroll
+    for (int r = 0; r < ITEMS; r++)
+    {
+        const unsigned p = r ? k[r ? r - 1 : 0] : prev;
+        if (k[r] != 0xffffffffu && ((r == 0 && tid == 0) || k[r] != p)) heads |= 1u << r;
+    }
+    int pos, total;
+    typename CtaSort<ITEMS>::Scan(temp.scan).ExclusiveSum(__popc(heads), pos, total);
+#pragma unroll
+    for (int r = 0; r < ITEMS; r++) if (heads >> r & 1) emit(pos++, (int)k[r]);
+    __syncthreads();
+    return total;
+}
+
+template <typename Load, typename Emit>
+__device__ __forceinline__ int cta_list(CtaTemp &temp, unsigned *last, int n, int bits, Load load, Emit emit)
+{
+    if (n <= 1024) return cta_sort_unique<4>(temp.t4, last, n, bits, load, emit);
+    return cta_sort_unique<16>(temp.t16, last, n, bits, load, emit);
+}
+
+// The same for any n by a CTA of 1024 threads with a bitmap of `words` (a multiple of 1024) shared 32-bit words: one pass
+// over the keys per words*32 columns.  A bitmap of all columns costs its own size, which for n > 4096 is less than sorting.
+template <typename Load, typename Emit>
+__device__ __forceinline__ int cta_bitmap_unique(unsigned *bm, int words, int *s_warp /* [33] */, int n, int colA, Load load, Emit emit)
+{
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, per_warp = words / 32;
+    int done = 0;
+    for (long long lo = 0; lo < colA; lo += (long long)words * 32)
+    {
+        for (int i = tid; i < words / 4; i += 1024) reinterpret_cast<uint4 *>(bm)[i] = make_uint4(0u, 0u, 0u, 0u);
+        __syncthreads();
+        const unsigned span = (unsigned)min((long long)words * 32, (long long)colA - lo), first = (unsigned)lo;
+#pragma unroll 4
+        for (int e = tid; e < n; e += 1024)
+        {
+            const unsigned c = (unsigned)load(e) - first;
+            if (c < span) atomicOr(&bm[c >> 5], 1u << (c & 31));
+        }
+        __syncthreads();
+        int sum = 0;
+        for (int i = lane; i < per_warp; i += 32) sum += __popc(bm[warp * per_warp + i]);
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (lane == 0) s_warp[warp] = sum;
+        __syncthreads();
+        if (warp == 0)
+        {
+            const int v = s_warp[lane];
+            int incl = v;
+            for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += y; }
+            s_warp[lane] = incl - v;
+            if (lane == 31) s_warp[32] = incl;
+        }
+        __syncthreads();
+        int run = done + s_warp[warp];
+        for (int i = lane; i < per_warp; i += 32)
+        {
+            unsigned w = bm[warp * per_warp + i];
+            const int c = __popc(w);
+            int incl = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += y; }
+            int pos = run + incl - c;
+            while (w) { emit(pos++, (int)(first + (unsigned)(warp * per_warp + i) * 32u + (unsigned)__ffs(w) - 1u)); w &= w - 1; }
+            run += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        done += s_warp[32];
+        __syncthreads();
+    }
+    return done;
+}
+
+// ---- step 1: lists of the 8-row blocks, and the consistency check of the CSR
+//
+// Row pointers must start at 0, never decrease and end at nnz, every column must lie in [0, colA).  A CSR that fails is
+// reported through stats->bad before anything is indexed with its contents (ranges used here are clamped to [0, nnz]).
+
+__device__ __forceinline__ void block_range(int b, int rowA, int nnz, const int *__restrict__ rowptr, int &begin, int &n)
+{
+    begin = min(max(rowptr[b * 8], 0), nnz);
+    n = min(max(rowptr[b * 8 + min(8, rowA - b * 8)], begin), nnz) - begin;
+}
+
+__global__ void __launch_bounds__(256) k_block_lists(int nb8, int rowA, int colA, int nnz, const int *__restrict__ rowptr, const int *__restrict__ colidx,
+                                                     int *__restrict__ ucols, int *__restrict__ ulen, int *__restrict__ mid, int *__restrict__ big, ConvStats *st)
+{
+    const int lane = threadIdx.x & 31, warps = (gridDim.x * blockDim.x) >> 5;
+    bool wrong = false;
+    for (int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; b < nb8 + 16; b += warps)
+    {
+        if (b >= nb8) { if (lane == 0) ulen[b] = 0; continue; }   // windows at the end look past the last block
+        const int r = b * 8 + lane;
+        int rb = 0, re = 0;
+        if (lane < 8 && r < rowA)
+        {
+            rb = rowptr[r]; re = rowptr[r + 1];
+            if (rb > re || rb < 0 || re > nnz || (r == 0 && rb != 0) || (r == rowA - 1 && re != nnz)) wrong = true;
+        }
+        const int begin = min(max(__shfl_sync(0xffffffffu, rb, 0), 0), nnz);
+        const int n = min(max(__shfl_sync(0xffffffffu, re, min(8, rowA - b * 8) - 1), begin), nnz) - begin;
+        if (n > SMALL_N)
+        {
+            if (lane == 0)
+            {
+                if (n <= MID_N) mid[atomicAdd(&st->n_mid[0], 1)] = b; else big[atomicAdd(&st->n_big[0], 1)] = b;
+            }
+            continue;
+        }
+        const int len = warp_list(n, lane,
+                                  [&](int e) { const int c = colidx[begin + e]; wrong |= c < 0 || c >= colA; return c; },
+                                  [&](int pos, int c) { ucols[begin + pos] = c; });
+        if (lane == 0) ulen[b] = len;
+    }
+    if (wrong) atomicExch(&st->bad, 1);
+}
+
+__global__ void __launch_bounds__(256) k_block_lists_mid(int rowA, int colA, int nnz, int bits, const int *__restrict__ rowptr, const int *__restrict__ colidx,
+                                                         int *__restrict__ ucols, int *__restrict__ ulen, const int *__restrict__ mid, ConvStats *st)
+{
+    __shared__ CtaTemp temp;
+    __shared__ unsigned last[256];
+    bool wrong = false;
+    const int count = st->n_mid[0];
+    for (int i = blockIdx.x; i < count; i += gridDim.x)
+    {
+        const int b = mid[i];
+        int begin, n;
+        block_range(b, rowA, nnz, rowptr, begin, n);
+        const int len = cta_list(temp, last, n, bits, [&](int e) { const int c = colidx[begin + e]; wrong |= c < 0 || c >= colA; return c; },
+                                 [&](int pos, int c) { ucols[begin + pos] = c; });
+        if (threadIdx.x == 0) ulen[b] = len;
+    }
+    if (wrong) atomicExch(&st->bad, 1);
+}
+
+__global__ void __launch_bounds__(1024) k_block_lists_big(int rowA, int colA, int nnz, int words, const int *__restrict__ rowptr, const int *__restrict__ colidx,
+                                                          int *__restrict__ ucols, int *__restrict__ ulen, const int *__restrict__ big, ConvStats *st)
+{
+    extern __shared__ __align__(16) unsigned bm[];
+    __shared__ int s_warp[33];
+    bool wrong = false;
+    const int count = st->n_big[0];
+    for (int i = blockIdx.x; i < count; i += gridDim.x)
+    {
+        const int b = big[i];
+        int begin, n;
+        block_range(b, rowA, nnz, rowptr, begin, n);
+        const int len = cta_bitmap_unique(bm, words, s_warp, n, colA, [&](int e) { const int c = colidx[begin + e]; wrong |= c < 0 || c >= colA; return c; },
+                                          [&](int pos, int c) { ucols[begin + pos] = c; });
+        if (threadIdx.x == 0) ulen[b] = len;
+    }
+    if (wrong) atomicExch(&st->bad, 1);
+}
+
+// ---- step 2: columns of a block that the previous q blocks do not hold
+//
+// Let p be the last block before j that holds column c of block j.  c counts in the window that starts at block b <= j
+// (and reaches j) exactly when p < b.  fresh[j][q] = number of columns of j with p < j - q, so a window of w blocks that
+// starts at b holds sum over q < w of fresh[b + q][q] distinct columns.
+
 __device__ __forceinline__ int lower_bound_dev(const int *a, int n, int key)
 {
     int lo = 0, hi = n;
     while (lo < hi)
     {
         int mid = (lo + hi) >> 1;
-        if (__ldg(a + mid) < key) lo = mid + 1; else hi = mid;
+        if (a[mid] < key) lo = mid + 1; else hi = mid;
     }
     return lo;
 }
 
-// ---- stage 1
-
-// Keys of all entries, and the consistency check of the CSR: row pointers start at 0, never decrease and end at nnz,
-// every column lies in [0, colA).  A CSR that fails is reported through *bad before anything is indexed with its
-// contents (the row ranges used here are clamped to [0, nnz]); every slot of keys[] is written for a valid CSR.
-__global__ void k_make_block_keys(int rowA, int colA, int nnz, const int *__restrict__ rowptr, const int *__restrict__ colidx,
-                                  unsigned long long *__restrict__ keys, int *__restrict__ bad)
+// distance to the last earlier block that holds c, at most `reach` blocks back; reach + 1 when there is none
+__device__ __forceinline__ int distance_back(int j, int c, int reach, int nnz, const int *__restrict__ rowptr, const int *__restrict__ ucols,
+                                             const int *__restrict__ ulen)
 {
-    const int lane = threadIdx.x & 31;
-    const int warps = (gridDim.x * blockDim.x) >> 5;
-    int wrong = 0;
-    for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rowA; r += warps)
+    for (int q = 1; q <= reach && q <= j; q++)
     {
-        int b = rowptr[r], e = rowptr[r + 1];
-        if (b > e || b < 0 || e > nnz || (r == 0 && b != 0) || (r == rowA - 1 && e != nnz)) wrong = 1;
-        b = min(max(b, 0), nnz); e = min(max(e, b), nnz);
-        const unsigned long long hi = (unsigned long long)(r >> 3) << 32;
-        for (int j = b + lane; j < e; j += 32)
+        const int len = ulen[j - q];
+        const int *list = ucols + min(max(rowptr[(j - q) * 8], 0), nnz);
+        if (len == 0 || c < list[0] || c > list[len - 1]) continue;
+        const int at = lower_bound_dev(list, len, c);
+        if (at < len && list[at] == c) return q;
+    }
+    return reach + 1;
+}
+
+// Blocks of up to SMALL_N entries: a warp each (the first `warp_ctas` CTAs).  Longer ones: a CTA each, from the lists of
+// step 1, so that a hub's list is not one warp's serial work.
+__global__ void __launch_bounds__(256) k_fresh_columns(int nb8, int rowA, int nnz, int reach, int warp_ctas, const int *__restrict__ rowptr,
+                                                       const int *__restrict__ ucols, const int *__restrict__ ulen, const int *__restrict__ mid,
+                                                       const int *__restrict__ big, const ConvStats *st, int *__restrict__ fresh)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if ((int)blockIdx.x < warp_ctas)
+    {
+        for (int j = blockIdx.x * 8 + warp; j < nb8 + 8; j += warp_ctas * 8)
         {
-            const int c = colidx[j];
-            if (c < 0 || c >= colA) wrong = 1;
-            keys[j] = hi | (unsigned int)c;
-        }
-    }
-    if (wrong) atomicExch(bad, 1);
-}
-
-// first index whose (key >> 32) >= g, for g = 0..ngroups (+ `pad` more entries holding the total)
-__global__ void k_group_offsets(const unsigned long long *__restrict__ keys, const int *__restrict__ n_ptr, int ngroups, int pad,
-                                int *__restrict__ ptr)
-{
-    int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g > ngroups + pad) return;
-    const int n = *n_ptr;
-    if (g > ngroups) { ptr[g] = n; return; }
-    int lo = 0, hi = n;
-    while (lo < hi)
-    {
-        int mid = (lo + hi) >> 1;
-        if ((int)(keys[mid] >> 32) < g) lo = mid + 1; else hi = mid;
-    }
-    ptr[g] = lo;
-}
-
-__global__ void k_low_words(const unsigned long long *__restrict__ keys, const int *__restrict__ n_ptr, int *__restrict__ out)
-{
-    const int n = *n_ptr;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = (int)(unsigned int)keys[i];
-}
-
-// ---- stage 2: distinct columns of windows of 2 and 8 consecutive blocks
-//
-// A column that occurs in block j counts once in every window [b, b+span) that contains j but not the previous block p
-// that holds the same column: b in (max(p, j-span), j].  So every (block, column) pair adds +1 at max(p, j-span)+1 and -1
-// at j+1 of a difference array, and a prefix sum gives the exact distinct count of every window.  The previous block of
-// every pair comes from one more radix sort, by (column, block).  Work is linear in the number of pairs, whatever the
-// row lengths (a warp per window with searches in the earlier lists took 39 ms on a scale-20 R-MAT graph; this takes 2).
-
-__global__ void k_col_block_keys(const unsigned long long *__restrict__ ukeys, int n, int block_bits, unsigned long long *__restrict__ out)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const unsigned long long k = ukeys[i];
-    out[i] = ((k & 0xffffffffull) << block_bits) | (k >> 32);
-}
-
-__global__ void k_window_diffs(const unsigned long long *__restrict__ by_col, int n, int block_bits, int want64, int *__restrict__ d16,
-                               int *__restrict__ d64)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const unsigned long long mask = (1ull << block_bits) - 1ull, k = by_col[i];
-    const int j = (int)(k & mask);
-    int p = -1;
-    if (i > 0)
-    {
-        const unsigned long long q = by_col[i - 1];
-        if ((q >> block_bits) == (k >> block_bits)) p = (int)(q & mask);
-    }
-    atomicAdd(&d16[max(p, j - 2) + 1], 1);
-    atomicAdd(&d16[j + 1], -1);
-    if (want64)
-    {
-        atomicAdd(&d64[max(p, j - 8) + 1], 1);
-        atomicAdd(&d64[j + 1], -1);
-    }
-}
-
-// ---- stage 3: the upstream decision at every 8-aligned start (src/hetero_split.h:196-276)
-
-__global__ void k_decide(int nb8, int rowA, float gamma, float delta, int fixed, const int *__restrict__ u8_ptr,
-                         const int *__restrict__ n16, const int *__restrict__ n64, unsigned char *__restrict__ cls_of)
-{
-    int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nb8) return;
-    if (fixed >= 0) { cls_of[b] = (unsigned char)fixed; return; }  // src/hetero_split.h:152-169
-    const long long i = (long long)b * 8;
-    int is64 = 0;
-    if (gamma < 4.0f && i + 64 <= rowA)
-    {
-        const int N64 = n64[b];
-        if (N64 > 0)
-        {
-            const float thr = gamma * N64;
-            int s16 = 0;
-            for (int q = 0; q < 4 && !is64; q++)
+            int mine = 0;   // lane q counts fresh[j][q]
+            if (j < nb8)
             {
-                s16 += n16[b + 2 * q];
-                if ((float)s16 > thr) is64 = 1;
+                int begin, n;
+                block_range(j, rowA, nnz, rowptr, begin, n);
+                if (n > SMALL_N) continue;
+                const int len = ulen[j];
+                for (int i = 0; i < len; i += 32)
+                {
+                    const bool on = i + lane < len;
+                    const int dist = on ? distance_back(j, ucols[begin + i + lane], reach, nnz, rowptr, ucols, ulen) : 0;
+                    for (int q = 0; q <= reach; q++)
+                    {
+                        const int c = __popc(__ballot_sync(0xffffffffu, on && dist > q));
+                        if (lane == q) mine += c;
+                    }
+                }
+            }
+            if (lane < 8) fresh[j * 8 + lane] = mine;
+        }
+        return;
+    }
+    __shared__ int s_cnt[8];
+    const int n_mid = st->n_mid[0], n_all = n_mid + st->n_big[0];
+    for (int i = (int)blockIdx.x - warp_ctas; i < n_all; i += (int)gridDim.x - warp_ctas)
+    {
+        const int j = i < n_mid ? mid[i] : big[i - n_mid];
+        if (threadIdx.x < 8) s_cnt[threadIdx.x] = 0;
+        __syncthreads();
+        const int begin = min(max(rowptr[j * 8], 0), nnz), len = ulen[j];
+        int mine = 0;
+        for (int t = warp * 32; t < len; t += 256)
+        {
+            const bool on = t + lane < len;
+            const int dist = on ? distance_back(j, ucols[begin + t + lane], reach, nnz, rowptr, ucols, ulen) : 0;
+            for (int q = 0; q <= reach; q++)
+            {
+                const int c = __popc(__ballot_sync(0xffffffffu, on && dist > q));
+                if (lane == q) mine += c;
             }
         }
+        if (lane < 8 && mine) atomicAdd(&s_cnt[lane], mine);
+        __syncthreads();
+        if (threadIdx.x < 8) fresh[j * 8 + threadIdx.x] = s_cnt[threadIdx.x];
+        __syncthreads();
     }
-    if (is64) { cls_of[b] = 0; return; }
-    int is16 = 0;
-    if (delta <= 0.0f) is16 = 1;
-    else if (!(delta > 2.0f) && i + 16 <= rowA)
-    {
-        const int N16 = n16[b];
-        if (N16 > 0)
-        {
-            const float thr = delta * N16;
-            int s8 = u8_ptr[b + 1] - u8_ptr[b];
-            if ((float)s8 >= thr) is16 = 1;
-            else
-            {
-                s8 += u8_ptr[b + 2] - u8_ptr[b + 1];
-                if ((float)s8 >= thr) is16 = 1;
-            }
-        }
-    }
-    cls_of[b] = is16 ? 1 : 2;
 }
+
+// ---- step 3: the upstream decision at every 8-aligned start (src/hetero_split.h:196-276) and the greedy chain
 
 __device__ __forceinline__ int step_of(int cls) { return cls == 0 ? 8 : (cls == 1 ? 2 : 1); }
 
-// The greedy chain i <- i + step(i) is resolved chunk-wise.  Chunks are short (CHAIN_L blocks) and staged in shared
-// memory, so that a walk costs shared-memory latency per step; the chunks are then linked by a parallel scan over
-// "entry offset -> exit offset" tables (8 states), not by a serial pass.
+constexpr int LOCAL_CHUNKS = 8;     // chunks per CTA of k_chain_local
+constexpr int EMIT_CHUNKS = 32;     // chunks per CTA of k_chain_emit
+constexpr int CHAIN_N = 9;          // panels, tiles and entries of the three classes
 
-// For every chunk of CHAIN_L blocks and every entry offset 0..7: where the chain leaves the chunk and how
-// many panels of each class it creates inside.  One thread per (chunk, entry); 32 chunks per block of 256 threads.
-__global__ void __launch_bounds__(256)
-k_chain_local(int nb8, int nchunk, const unsigned char *__restrict__ cls_of, unsigned char *__restrict__ exit_off,
-              int *__restrict__ counts /* [nchunk*8][3] */)
+// The chain i <- i + step(i) is resolved chunk-wise.  Chunks are short (CHAIN_L blocks) and staged in shared memory, so
+// that a walk costs shared-memory latency per step; the chunks are then linked by a parallel scan over "entry offset ->
+// exit offset" tables (8 states), not by a serial pass.
+//
+// This kernel: the class every start would take and the tiles its panel would have; then, for every chunk and every entry
+// offset 0..7, where the chain leaves the chunk and how many panels, tiles and entries of each class it passes.
+__global__ void __launch_bounds__(LOCAL_CHUNKS * 8)
+k_chain_local(int nb8, int nchunk, int rowA, int nnz, int precision, float gamma, float delta, int fixed, int reach, const int *__restrict__ rowptr,
+              const int *__restrict__ ulen, const int *__restrict__ fresh, unsigned char *__restrict__ cls_of, int *__restrict__ tiles_of,
+              unsigned char *__restrict__ exit_off, int *__restrict__ counts /* [nchunk*8][CHAIN_N] */)
 {
-    __shared__ unsigned char cls_s[32 * CHAIN_L];
-    const long long first = (long long)blockIdx.x * 32 * CHAIN_L;
-    for (int i = threadIdx.x; i < 32 * CHAIN_L; i += 256) cls_s[i] = first + i < nb8 ? cls_of[first + i] : 2;
+    constexpr int NB = LOCAL_CHUNKS * CHAIN_L;
+    __shared__ int n16_s[NB + 8], rp_s[NB + 9], tiles_s[NB];
+    __shared__ unsigned char cls_s[NB];
+    const int first = blockIdx.x * NB, tid = threadIdx.x;
+    for (int i = tid; i < NB + 9; i += LOCAL_CHUNKS * 8)
+    {
+        const int b = first + i;
+        rp_s[i] = min(max(rowptr[b < nb8 ? b * 8 : rowA], 0), nnz);
+        if (i < NB + 8 && reach > 0) n16_s[i] = b < nb8 ? fresh[b * 8] + fresh[b * 8 + 9] : 0;
+    }
     __syncthreads();
-    const int t = blockIdx.x * 256 + threadIdx.x;
+    for (int i = tid; i < NB; i += LOCAL_CHUNKS * 8)
+    {
+        const int b = first + i;
+        if (b >= nb8) break;
+        const long long row = (long long)b * 8;
+        int N64 = 0;
+        if (reach == 7)
+#pragma unroll
+            for (int q = 0; q < 8; q++) N64 += b + q < nb8 ? fresh[(b + q) * 8 + q] : 0;
+        int k = 2;
+        if (fixed >= 0) k = fixed;   // src/hetero_split.h:152-169
+        else
+        {
+            bool is64 = false;
+            if (gamma < 4.0f && row + 64 <= rowA && N64 > 0)
+            {
+                const float thr = gamma * N64;
+                int s16 = 0;
+                for (int q = 0; q < 4 && !is64; q++)
+                {
+                    s16 += n16_s[i + 2 * q];
+                    if ((float)s16 > thr) is64 = true;
+                }
+            }
+            if (is64) k = 0;
+            else if (delta <= 0.0f) k = 1;
+            else if (!(delta > 2.0f) && row + 16 <= rowA && n16_s[i] > 0)
+            {
+                const float thr = delta * n16_s[i];
+                int s8 = ulen[b];
+                bool is16 = (float)s8 >= thr;
+                if (!is16) { s8 += ulen[b + 1]; is16 = (float)s8 >= thr; }
+                if (is16) k = 1;
+            }
+        }
+        const int d = k == 0 ? N64 : (k == 1 ? n16_s[i] : ulen[b]), bn = tsp_bn(precision, k);
+        cls_s[i] = (unsigned char)k; tiles_s[i] = (d + bn - 1) / bn;   // src/csr2tile.h:45-46
+        cls_of[b] = (unsigned char)k; tiles_of[b] = tiles_s[i];
+    }
+    __syncthreads();
+    const int t = blockIdx.x * LOCAL_CHUNKS * 8 + tid;
     if (t >= nchunk * 8) return;
-    const int c = t >> 3, o = t & 7, lc = threadIdx.x >> 3;
-    const int len = (int)min((long long)CHAIN_L, (long long)nb8 - (long long)c * CHAIN_L);
-    int pos = o, cnt[3] = {0, 0, 0};
+    const int c = t >> 3, o = t & 7, base = (tid >> 3) * CHAIN_L;
+    const int len = min(CHAIN_L, nb8 - c * CHAIN_L);
+    int pos = o, cnt[CHAIN_N] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     while (pos < len)
     {
-        const int k = cls_s[lc * CHAIN_L + pos];
-        cnt[k]++;
-        pos += step_of(k);
+        const int k = cls_s[base + pos], st = step_of(k), tl = tiles_s[base + pos], en = rp_s[base + pos + st] - rp_s[base + pos];
+#pragma unroll
+        for (int q = 0; q < 3; q++) if (q == k) { cnt[q]++; cnt[3 + q] += tl; cnt[6 + q] += en; }
+        pos += st;
     }
     const int off = pos - CHAIN_L;
     exit_off[t] = (unsigned char)(off < 0 ? 0 : (off > 7 ? 7 : off));
-    counts[t * 3 + 0] = cnt[0]; counts[t * 3 + 1] = cnt[1]; counts[t * 3 + 2] = cnt[2];
+#pragma unroll
+    for (int q = 0; q < CHAIN_N; q++) counts[t * CHAIN_N + q] = cnt[q];
 }
 
 // Links the chunks: the entry offset of every chunk (composition of the chunks' transition tables, 8 states of 3 bits
-// packed into one word) and the number of panels of each class before it.  One block; scans by composition.
+// packed into one word) and the panels, tiles and entries of each class before it.  One block; scans by composition.
 __global__ void __launch_bounds__(1024)
 k_chain_compose(int nchunk, const unsigned char *__restrict__ exit_off, const int *__restrict__ counts, int *__restrict__ entry,
-                int *__restrict__ base /* [nchunk+1][3] */)
+                int *__restrict__ base /* [nchunk][CHAIN_N] */, ConvStats *st)
 {
     __shared__ unsigned int warp_f[32];
-    __shared__ int warp_n[32][3];
+    __shared__ int warp_n[32][CHAIN_N];
     __shared__ unsigned int carry_state;
-    __shared__ int carry_n[3];
+    __shared__ int carry_n[CHAIN_N];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // f(state) for all 8 states in one word; compose(f, g)(x) = g(f(x)) -- f first
     auto apply = [](unsigned int f, unsigned int x) { return (f >> (3 * x)) & 7u; };
@@ -276,7 +557,8 @@ k_chain_compose(int nchunk, const unsigned char *__restrict__ exit_off, const in
         return h;
     };
     constexpr unsigned int IDENT = 0u | 1u << 3 | 2u << 6 | 3u << 9 | 4u << 12 | 5u << 15 | 6u << 18 | 7u << 21;
-    if (threadIdx.x == 0) { carry_state = 0; carry_n[0] = carry_n[1] = carry_n[2] = 0; }
+    if (threadIdx.x == 0) carry_state = 0;
+    if (threadIdx.x < CHAIN_N) carry_n[threadIdx.x] = 0;
     __syncthreads();
     for (int base_c = 0; base_c < nchunk; base_c += 1024)
     {
@@ -284,8 +566,9 @@ k_chain_compose(int nchunk, const unsigned char *__restrict__ exit_off, const in
         unsigned int f = IDENT;
         if (c < nchunk)
         {
+            const uint2 w = *reinterpret_cast<const uint2 *>(exit_off + (size_t)c * 8);
             f = 0;
-            for (unsigned int x = 0; x < 8; x++) f |= (unsigned int)exit_off[c * 8 + x] << (3 * x);
+            for (unsigned int x = 0; x < 8; x++) f |= (((x < 4 ? w.x : w.y) >> (8 * (x & 3))) & 7u) << (3 * x);
         }
         // inclusive scan of the transition tables over the 1024 chunks of this pass
         unsigned int incl = f;
@@ -304,92 +587,111 @@ k_chain_compose(int nchunk, const unsigned char *__restrict__ exit_off, const in
         if (lane == 0) excl = IDENT;
         if (warp > 0) excl = compose(warp_f[warp - 1], excl);
         const unsigned int e = apply(excl, carry_state);       // the true entry offset of chunk c
-        int n[3] = {0, 0, 0};
-        if (c < nchunk)
+        int n[CHAIN_N], in[CHAIN_N];
+#pragma unroll
+        for (int k = 0; k < CHAIN_N; k++) n[k] = c < nchunk ? counts[(c * 8 + (int)e) * CHAIN_N + k] : 0;
+        if (c < nchunk) entry[c] = (int)e;
+        // exclusive prefix sums along the true path
+#pragma unroll
+        for (int k = 0; k < CHAIN_N; k++)
         {
-            entry[c] = (int)e;
-            const int t = c * 8 + (int)e;
-            n[0] = counts[t * 3 + 0]; n[1] = counts[t * 3 + 1]; n[2] = counts[t * 3 + 2];
+            in[k] = n[k];
+            for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, in[k], o); if (lane >= o) in[k] += y; }
+            if (lane == 31) warp_n[warp][k] = in[k];
         }
-        // exclusive prefix sums of the panel counts along the true path
-        int in[3] = {n[0], n[1], n[2]};
-        for (int o = 1; o < 32; o <<= 1)
-#pragma unroll
-            for (int k = 0; k < 3; k++) { const int y = __shfl_up_sync(0xffffffffu, in[k], o); if (lane >= o) in[k] += y; }
-        if (lane == 31) { warp_n[warp][0] = in[0]; warp_n[warp][1] = in[1]; warp_n[warp][2] = in[2]; }
         __syncthreads();
-        if (warp == 0)
+        if (warp < CHAIN_N)
         {
-            int w[3] = {warp_n[lane][0], warp_n[lane][1], warp_n[lane][2]};
-            for (int o = 1; o < 32; o <<= 1)
-#pragma unroll
-                for (int k = 0; k < 3; k++) { const int y = __shfl_up_sync(0xffffffffu, w[k], o); if (lane >= o) w[k] += y; }
-            warp_n[lane][0] = w[0]; warp_n[lane][1] = w[1]; warp_n[lane][2] = w[2];
+            int w = warp_n[lane][warp];
+            for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, w, o); if (lane >= o) w += y; }
+            warp_n[lane][warp] = w;
         }
         __syncthreads();
         if (c < nchunk)
 #pragma unroll
-            for (int k = 0; k < 3; k++) base[c * 3 + k] = carry_n[k] + (warp ? warp_n[warp - 1][k] : 0) + in[k] - n[k];
+            for (int k = 0; k < CHAIN_N; k++) base[c * CHAIN_N + k] = carry_n[k] + (warp ? warp_n[warp - 1][k] : 0) + in[k] - n[k];
         __syncthreads();
         if (threadIdx.x == 1023)   // totals of this pass -> carry for the next
         {
             carry_state = apply(compose(excl, f), carry_state);
 #pragma unroll
-            for (int k = 0; k < 3; k++) carry_n[k] += warp_n[31][k];
+            for (int k = 0; k < CHAIN_N; k++) carry_n[k] += warp_n[31][k];
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) { base[nchunk * 3 + 0] = carry_n[0]; base[nchunk * 3 + 1] = carry_n[1]; base[nchunk * 3 + 2] = carry_n[2]; }
-}
-
-// Walk every chunk from its true entry and emit the panels in scan order.  One thread per chunk, 128 chunks per block.
-__global__ void __launch_bounds__(128)
-k_chain_emit(int nb8, int nchunk, int rowA, const unsigned char *__restrict__ cls_of, const int *__restrict__ entry,
-             const int *__restrict__ base, const int *__restrict__ rowptr, int *__restrict__ seq_blk,
-             unsigned char *__restrict__ seq_cls, int *__restrict__ seq_idx, int *__restrict__ blk_seq,
-             unsigned long long *__restrict__ class_rows_nnz /* [3][2] */)
-{
-    __shared__ unsigned char cls_s[128 * CHAIN_L];
-    const long long first = (long long)blockIdx.x * 128 * CHAIN_L;
-    for (int i = threadIdx.x; i < 128 * CHAIN_L; i += 128) cls_s[i] = first + i < nb8 ? cls_of[first + i] : 2;
-    __syncthreads();
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= nchunk) return;
-    long long pos = (long long)c * CHAIN_L + entry[c];
-    const long long end = min((long long)(c + 1) * CHAIN_L, (long long)nb8);
-    int idx[3] = {base[c * 3 + 0], base[c * 3 + 1], base[c * 3 + 2]};
-    int seq = idx[0] + idx[1] + idx[2];
-    unsigned long long rows[3] = {0, 0, 0}, nnz[3] = {0, 0, 0};
-    while (pos < end)
+    if (threadIdx.x < 3)
     {
-        const int k = cls_s[pos - first], st = step_of(k);
-        seq_blk[seq] = (int)pos;
-        seq_cls[seq] = (unsigned char)k;
-        seq_idx[seq] = idx[k]++;
-        for (int q = 0; q < st && pos + q < nb8; q++) blk_seq[pos + q] = seq;
-        const long long r0 = pos * 8, r1 = min(r0 + st * 8, (long long)rowA);
-        rows[k] += (unsigned long long)(r1 - r0);
-        nnz[k] += (unsigned long long)(rowptr[r1] - rowptr[r0]);
-        seq++;
-        pos += st;
+        st->panels[threadIdx.x] = carry_n[threadIdx.x];
+        st->tiles[threadIdx.x] = carry_n[3 + threadIdx.x];
+        st->nnz[threadIdx.x] = carry_n[6 + threadIdx.x];
     }
-    for (int k = 0; k < 3; k++)
-        if (rows[k])
-        {
-            atomicAdd(&class_rows_nnz[k * 2 + 0], rows[k]);
-            atomicAdd(&class_rows_nnz[k * 2 + 1], nnz[k]);
-        }
 }
 
-// ---- stage 4
-
-__global__ void k_make_panel_keys(const unsigned long long *__restrict__ ukeys, int n, const int *__restrict__ blk_seq,
-                                  unsigned long long *__restrict__ out)
+// Per-class arrays of the whole matrix, in the workspace (a shard copies its slice): first tile and first entry of every
+// panel (one past the last = totals) and its first row.
+struct ClassArrays
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const unsigned long long k = ukeys[i];
-    out[i] = ((unsigned long long)blk_seq[(int)(k >> 32)] << 32) | (k & 0xffffffffull);
+    int *tile_ptr[3], *nnz_ptr[3], *panel_row[3];
+};
+// The panels in scan order, written only for sharded conversions: block, class, index inside the class, tiles.
+struct SeqArrays
+{
+    int *blk, *idx, *tiles;
+    unsigned char *cls;
+};
+
+// Walks every chunk from its true entry and writes its panels.  One thread per chunk, 32 chunks per CTA.
+__global__ void __launch_bounds__(128)
+k_chain_emit(int nb8, int nchunk, int rowA, int nnz, const unsigned char *__restrict__ cls_of, const int *__restrict__ tiles_of,
+             const int *__restrict__ entry, const int *__restrict__ base, const int *__restrict__ rowptr, ClassArrays out, SeqArrays seq, ConvStats *st)
+{
+    constexpr int NB = EMIT_CHUNKS * CHAIN_L;
+    __shared__ unsigned char cls_s[NB];
+    __shared__ int tiles_s[NB], rp_s[NB + 8];
+    __shared__ int hist_s[3][TSP_HIST_BINS], max_s[3];
+    const int first = blockIdx.x * NB, tid = threadIdx.x;
+    for (int i = tid; i < NB + 8; i += 128)
+    {
+        const int b = first + i;
+        if (i < NB) { cls_s[i] = b < nb8 ? cls_of[b] : 2; tiles_s[i] = b < nb8 ? tiles_of[b] : 0; }
+        rp_s[i] = min(max(rowptr[b < nb8 ? b * 8 : rowA], 0), nnz);
+    }
+    for (int i = tid; i < 3 * TSP_HIST_BINS; i += 128) (&hist_s[0][0])[i] = 0;
+    if (tid < 3) max_s[tid] = 0;
+    __syncthreads();
+    const int c = blockIdx.x * EMIT_CHUNKS + tid;
+    if (tid < EMIT_CHUNKS && c < nchunk)
+    {
+        int at[CHAIN_N];
+#pragma unroll
+        for (int q = 0; q < CHAIN_N; q++) at[q] = base[c * CHAIN_N + q];
+        int pos = c * CHAIN_L + entry[c], sq = at[0] + at[1] + at[2];
+        const int end = min((c + 1) * CHAIN_L, nb8);
+        while (pos < end)
+        {
+            const int k = cls_s[pos - first], step = step_of(k), tl = tiles_s[pos - first], en = rp_s[pos - first + step] - rp_s[pos - first];
+#pragma unroll
+            for (int q = 0; q < 3; q++)
+                if (q == k)
+                {
+                    out.tile_ptr[q][at[q]] = at[3 + q]; out.nnz_ptr[q][at[q]] = at[6 + q]; out.panel_row[q][at[q]] = pos * 8;
+                    if (seq.blk) { seq.blk[sq] = pos; seq.cls[sq] = (unsigned char)q; seq.idx[sq] = at[q]; seq.tiles[sq] = tl; }
+                    at[q]++; at[3 + q] += tl; at[6 + q] += en;
+                }
+            const int len = min(max(tl, 0), TSP_HIST_BINS - 1);
+            atomicAdd(&hist_s[k][len], 1);
+            atomicMax(&max_s[k], tl);
+            sq++;
+            pos += step;
+            if (pos >= nb8) st->last_cls = k;
+        }
+        if (c == nchunk - 1)
+#pragma unroll
+            for (int q = 0; q < 3; q++) { out.tile_ptr[q][at[q]] = at[3 + q]; out.nnz_ptr[q][at[q]] = at[6 + q]; }
+    }
+    __syncthreads();
+    for (int i = tid; i < 3 * TSP_HIST_BINS; i += 128) { const int v = (&hist_s[0][0])[i]; if (v) atomicAdd(&(&st->hist[0][0])[i], v); }
+    if (tid < 3 && max_s[tid]) atomicMax(&st->max_len[tid], max_s[tid]);
 }
 
 // ---- shard selection on the device: a contiguous range of the panel sequence, balanced by tile bytes
@@ -439,68 +741,169 @@ __global__ void k_shard_bounds(const int *cuts, const unsigned char *__restrict_
     }
 }
 
-// rows and stored entries of every class inside the shard
-__global__ void k_class_totals(int s0, int s1, int rowA, const unsigned char *__restrict__ seq_cls, const int *__restrict__ seq_blk,
-                               const int *__restrict__ rowptr, unsigned long long *__restrict__ rows_nnz /* [3][2] */)
+// ---- step 4: this handle's share of the per-class arrays
+
+// d_tile_ptr and d_panel_row of all classes from the workspace arrays, panels [p0, p1) of every class
+__global__ void k_class_slices(ClassArrays all, int3 p0, int3 p1, ClassArrays mine, int *tn64, int *tn16, int *tn8)
 {
-    unsigned long long rows[3] = {0, 0, 0}, nnz[3] = {0, 0, 0};
-    for (int s = s0 + blockIdx.x * blockDim.x + threadIdx.x; s < s1; s += gridDim.x * blockDim.x)
-    {
-        const int k = seq_cls[s];
-        const long long r0 = (long long)seq_blk[s] * 8, r1 = min(r0 + tsp_bm(k), (long long)rowA);
-        rows[k] += (unsigned long long)(r1 - r0);
-        nnz[k] += (unsigned long long)(rowptr[r1] - rowptr[r0]);
-    }
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+#pragma unroll
     for (int k = 0; k < 3; k++)
-        if (rows[k]) { atomicAdd(&rows_nnz[k * 2], rows[k]); atomicAdd(&rows_nnz[k * 2 + 1], nnz[k]); }
-}
-
-__global__ void k_seq_tiles(int nseq, const int *__restrict__ pptr, const unsigned char *__restrict__ seq_cls, int precision,
-                            int *__restrict__ seq_tiles)
-{
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nseq) return;
-    const int bn = tsp_bn(precision, seq_cls[s]);
-    seq_tiles[s] = (pptr[s + 1] - pptr[s] + bn - 1) / bn;  // src/csr2tile.h:45-46
-}
-
-// scatter the per-panel tile counts and first rows of the shard [s0, s1) into the per-class arrays
-__global__ void k_class_arrays(int s0, int s1, const int *__restrict__ seq_tiles, const unsigned char *__restrict__ seq_cls,
-                               const int *__restrict__ seq_idx, const int *__restrict__ seq_blk, int p0_64, int p0_16, int p0_8,
-                               int *cnt64, int *cnt16, int *cnt8, int *row64, int *row16, int *row8)
-{
-    int s = s0 + blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= s1) return;
-    const int k = seq_cls[s];
-    const int p = seq_idx[s] - (k == 0 ? p0_64 : (k == 1 ? p0_16 : p0_8));
-    (k == 0 ? cnt64 : (k == 1 ? cnt16 : cnt8))[p] = seq_tiles[s];
-    (k == 0 ? row64 : (k == 1 ? row16 : row8))[p] = seq_blk[s] * 8;
-}
-
-// tile_colidx: sorted distinct columns, the tail padded with the panel's last column (src/csr2tile.h:117-132)
-__global__ void k_fill_colidx(int s0, int s1, int precision, const int *__restrict__ pptr, const int *__restrict__ pcols,
-                              const unsigned char *__restrict__ seq_cls, const int *__restrict__ seq_idx, int p0_64, int p0_16, int p0_8,
-                              const int *__restrict__ tp64, const int *__restrict__ tp16, const int *__restrict__ tp8,
-                              int *__restrict__ ci64, int *__restrict__ ci16, int *__restrict__ ci8)
-{
-    const int lane = threadIdx.x & 31;
-    const int warps = (gridDim.x * blockDim.x) >> 5;
-    for (int s = s0 + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); s < s1; s += warps)
     {
-        const int k = seq_cls[s], bn = tsp_bn(precision, k);
-        const int p = seq_idx[s] - (k == 0 ? p0_64 : (k == 1 ? p0_16 : p0_8));
-        const int *tp = k == 0 ? tp64 : (k == 1 ? tp16 : tp8);
-        int *ci = k == 0 ? ci64 : (k == 1 ? ci16 : ci8);
-        const int t0 = tp[p], nt = tp[p + 1] - t0;
-        if (nt == 0) continue;
-        const int g0 = pptr[s], d = pptr[s + 1] - g0;
-        const int last = pcols[g0 + d - 1];
-        int *dst = ci + (size_t)t0 * bn;
-        for (int q = lane; q < nt * bn; q += 32) dst[q] = q < d ? pcols[g0 + q] : last;
+        const int a = k == 0 ? p0.x : (k == 1 ? p0.y : p0.z), n = (k == 0 ? p1.x : (k == 1 ? p1.y : p1.z)) - a;
+        if (i > n) continue;
+        mine.tile_ptr[k][i] = all.tile_ptr[k][a + i] - all.tile_ptr[k][a];
+        if (i < n) mine.panel_row[k][i] = all.panel_row[k][a + i];
+        else (k == 0 ? tn64 : (k == 1 ? tn16 : tn8))[mine.tile_ptr[k][n]] = all.nnz_ptr[k][a + n] - all.nnz_ptr[k][a];   // total after the last tile
     }
 }
 
-// ---- stage 5: values and per-tile entry counts, one warp per original row
+// sharded conversions: tiles, entries and the panel-length histogram of panels [p0, p1) of every class
+__global__ void k_shard_stats(ClassArrays all, int3 p0, int3 p1, ConvStats *st)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+    {
+        const int a = k == 0 ? p0.x : (k == 1 ? p0.y : p0.z), n = (k == 0 ? p1.x : (k == 1 ? p1.y : p1.z)) - a;
+        if (i == 0) { st->tiles[k] = all.tile_ptr[k][a + n] - all.tile_ptr[k][a]; st->nnz[k] = all.nnz_ptr[k][a + n] - all.nnz_ptr[k][a]; }
+        if (i >= n) continue;
+        const int len = all.tile_ptr[k][a + i + 1] - all.tile_ptr[k][a + i];
+        atomicAdd(&st->hist[k][min(len, TSP_HIST_BINS - 1)], 1);
+        atomicMax(&st->max_len[k], len);
+    }
+}
+
+// ---- step 5: column lists of tall panels from the lists of their 8-row blocks
+
+// What the conversion kernels of one class work on.  nnz_ptr is the workspace array from this shard's first panel on.
+struct ClassView
+{
+    int cls, tilem;
+    const int *tile_ptr, *panel_row, *nnz_ptr;
+    int *tile_colidx, *tile_nnz;
+    int2 *items;      // {panel, slice} work list
+    int item_cap;
+};
+
+// entries and tiles up to which one warp builds a 16- or 8-row panel; the 16-row TF32 tiles are twice as large
+__host__ __device__ constexpr int small_cols(int precision, int cls) { return precision == 1 && cls == 1 ? 256 : 512; }
+__device__ __forceinline__ bool small_panel(int precision, int cls, int n, int nt) { return n <= SMALL_N && nt * tsp_bn(precision, cls) <= small_cols(precision, cls); }
+
+__device__ __forceinline__ void push_slices(const ClassView &v, int precision, int p, int nt, ConvStats *st)
+{
+    const int per = SLICE_COLS / tsp_bn(precision, v.cls), ns = (nt + per - 1) / per;
+    const int at = atomicAdd(&st->n_items[v.cls], ns);
+    for (int s = 0; s < ns && at + s < v.item_cap; s++) v.items[at + s] = make_int2(p, s);
+}
+
+// the up to eight block lists of a panel as one list of keys
+struct Segments
+{
+    int pre[9], start[8];
+    __device__ __forceinline__ int find(int e) const
+    {
+        int q = 0;
+#pragma unroll
+        for (int i = 1; i < 8; i++) q += e >= pre[i];
+        return start[q] + e - pre[q];
+    }
+};
+// filled by one warp; returns the number of keys
+__device__ __forceinline__ int load_segments(Segments &sg, int row0, int cls, int nb8, const int *__restrict__ rowptr, const int *__restrict__ ulen, int lane)
+{
+    const int q = lane & 7, b = row0 / 8 + q;
+    const bool on = lane < 8 && q < step_of(cls) && b < nb8;
+    const int len = on ? ulen[b] : 0, start = on ? rowptr[b * 8] : 0;
+    int incl = len;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += y; }
+    if (lane < 8) { sg.pre[lane] = incl - len; sg.start[lane] = start; }
+    if (lane == 7) sg.pre[8] = incl;
+    __syncwarp();
+    return __shfl_sync(0xffffffffu, incl, 7);
+}
+
+// A warp per panel of the 64-row class and per 16-row panel that is too long for k_fill_small; lists longer than SMALL_N
+// go to the CTA kernels below.  Also cuts the panels into work items.
+__global__ void __launch_bounds__(256) k_panel_lists(int nb8, int rowA, int precision, const int *__restrict__ rowptr, const int *__restrict__ ucols,
+                                                     const int *__restrict__ ulen, ClassView v64, ClassView v16, int2 *chunks, int chunk_cap,
+                                                     int *__restrict__ mid, int *__restrict__ big, ConvStats *st)
+{
+    __shared__ Segments segs[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = gridDim.x * 8;
+    for (int i = blockIdx.x * 8 + warp; i < v64.tilem + v16.tilem; i += warps)
+    {
+        const ClassView &v = i < v64.tilem ? v64 : v16;
+        const int p = i < v64.tilem ? i : i - v64.tilem, bm = tsp_bm(v.cls), bn = tsp_bn(precision, v.cls);
+        const int row0 = v.panel_row[p], t0 = v.tile_ptr[p], nt = v.tile_ptr[p + 1] - t0, n = rowptr[row0 + min(bm, rowA - row0)] - rowptr[row0];
+        if (nt == 0 || (v.cls == 1 && small_panel(precision, 1, n, nt))) continue;
+        const int keys = load_segments(segs[warp], row0, v.cls, nb8, rowptr, ulen, lane);
+        if (lane == 0)
+        {
+            push_slices(v, precision, p, nt, st);
+            if (v.cls == 0)
+            {
+                const int nc = (n + CHUNK_N - 1) / CHUNK_N, at = atomicAdd(&st->n_chunks, nc);
+                for (int s = 0; s < nc && at + s < chunk_cap; s++) chunks[at + s] = make_int2(p, s);
+            }
+            if (keys > SMALL_N) { if (keys <= MID_N) mid[atomicAdd(&st->n_mid[1], 1)] = i; else big[atomicAdd(&st->n_big[1], 1)] = i; }
+        }
+        if (keys > SMALL_N) { __syncwarp(); continue; }
+        int *dst = v.tile_colidx + (size_t)t0 * bn;
+        const int d = warp_list(keys, lane, [&](int e) { return ucols[segs[warp].find(e)]; }, [&](int pos, int c) { dst[pos] = c; });
+        __syncwarp();
+        const int last = dst[d - 1];
+        for (int q = d + lane; q < nt * bn; q += 32) dst[q] = last;   // src/csr2tile.h:117-132
+        __syncwarp();
+    }
+}
+
+__global__ void __launch_bounds__(256) k_panel_lists_mid(int nb8, int precision, int bits, const int *__restrict__ rowptr, const int *__restrict__ ucols,
+                                                         const int *__restrict__ ulen, ClassView v64, ClassView v16, const int *__restrict__ mid, const ConvStats *st)
+{
+    __shared__ CtaTemp temp;
+    __shared__ unsigned last_s[256];
+    __shared__ Segments sg;
+    const int count = st->n_mid[1];
+    for (int w = blockIdx.x; w < count; w += gridDim.x)
+    {
+        const int i = mid[w];
+        const ClassView &v = i < v64.tilem ? v64 : v16;
+        const int p = i < v64.tilem ? i : i - v64.tilem, bn = tsp_bn(precision, v.cls), t0 = v.tile_ptr[p], nt = v.tile_ptr[p + 1] - t0;
+        if (threadIdx.x < 32) load_segments(sg, v.panel_row[p], v.cls, nb8, rowptr, ulen, threadIdx.x);
+        __syncthreads();
+        int *dst = v.tile_colidx + (size_t)t0 * bn;
+        const int d = cta_list(temp, last_s, sg.pre[8], bits, [&](int e) { return ucols[sg.find(e)]; }, [&](int pos, int c) { dst[pos] = c; });
+        const int last = dst[d - 1];
+        for (int q = d + threadIdx.x; q < nt * bn; q += 256) dst[q] = last;
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(1024) k_panel_lists_big(int nb8, int colA, int precision, int words, const int *__restrict__ rowptr, const int *__restrict__ ucols,
+                                                          const int *__restrict__ ulen, ClassView v64, ClassView v16, const int *__restrict__ big, const ConvStats *st)
+{
+    extern __shared__ __align__(16) unsigned bm[];
+    __shared__ int s_warp[33];
+    __shared__ Segments sg;
+    const int count = st->n_big[1];
+    for (int w = blockIdx.x; w < count; w += gridDim.x)
+    {
+        const int i = big[w];
+        const ClassView &v = i < v64.tilem ? v64 : v16;
+        const int p = i < v64.tilem ? i : i - v64.tilem, bn = tsp_bn(precision, v.cls), t0 = v.tile_ptr[p], nt = v.tile_ptr[p + 1] - t0;
+        if (threadIdx.x < 32) load_segments(sg, v.panel_row[p], v.cls, nb8, rowptr, ulen, threadIdx.x);
+        __syncthreads();
+        int *dst = v.tile_colidx + (size_t)t0 * bn;
+        const int d = cta_bitmap_unique(bm, words, s_warp, sg.pre[8], colA, [&](int e) { return ucols[sg.find(e)]; }, [&](int pos, int c) { dst[pos] = c; });
+        const int last = dst[d - 1];
+        for (int q = d + threadIdx.x; q < nt * bn; q += 1024) dst[q] = last;
+        __syncthreads();
+    }
+}
+
+// ---- step 6: tiles of the 16- and 8-row classes
 
 template <typename V>
 __device__ __forceinline__ V add_in_value_type(V a, V b);
@@ -533,92 +936,292 @@ __device__ __forceinline__ void add_in_csr_order(V *vals, unsigned long long pos
     __syncwarp();
 }
 
-// One warp per original row: tile and slot of every entry; per-tile entry counts (all classes); dense tile values of
-// the 16- and 8-row classes; row masks of the 64-row tiles.
-template <typename V>
-__global__ void k_place_values(int rowA, int precision, int s0, int s1, const int *__restrict__ rowptr, const int *__restrict__ colidx,
-                               const V *__restrict__ val, const int *__restrict__ blk_seq, const unsigned char *__restrict__ seq_cls,
-                               const int *__restrict__ seq_idx, const int *__restrict__ seq_blk, const int *__restrict__ pptr,
-                               const int *__restrict__ pcols, int p0_64, int p0_16, int p0_8, const int *__restrict__ tp64,
-                               const int *__restrict__ tp16, const int *__restrict__ tp8, int *tn64, int *tn16, int *tn8,
-                               unsigned int *__restrict__ mask64 /* 32-bit words of the row masks */, V *v16, V *v8)
+
+// the row of a panel that entry j belongs to: largest r with rp[r] <= j (BM rows, a power of two)
+template <int BM>
+__device__ __forceinline__ int row_of(const int *rp, int j)
 {
-    const int lane = threadIdx.x & 31;
-    const int warps = (gridDim.x * blockDim.x) >> 5;
-    for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rowA; r += warps)
+    int r = 0;
+#pragma unroll
+    for (int s = BM / 2; s > 0; s >>= 1) if (j >= rp[r + s]) r += s;
+    return r;
+}
+template <typename V, int CLS>
+struct SmallFill
+{
+    static constexpr int PREC = sizeof(V) == 4 ? 1 : 0, BM = CLS == 1 ? 16 : 8, BN = PREC ? 8 : 16, COLS = small_cols(PREC, CLS), TILES = COLS / BN;
+    static constexpr int WARPS = 4;
+    struct Warp
     {
-        const int s = blk_seq[r >> 3];
-        if (s < s0 || s >= s1) continue;
-        const int jb = rowptr[r], je = rowptr[r + 1];
-        if (jb == je) continue;
-        const int k = seq_cls[s], bm = tsp_bm(k), bn = tsp_bn(precision, k);
-        const int p = seq_idx[s] - (k == 0 ? p0_64 : (k == 1 ? p0_16 : p0_8));
-        const int t0 = (k == 0 ? tp64 : (k == 1 ? tp16 : tp8))[p];
-        int *tn = k == 0 ? tn64 : (k == 1 ? tn16 : tn8);
-        V *vals = k == 1 ? v16 : v8;
-        const int ri = r - seq_blk[s] * 8;
-        const int g0 = pptr[s], d = pptr[s + 1] - g0;
-        for (int base = jb; base < je; base += 32)
+        V image[TILES * BM * BN];
+        int list[COLS];
+        unsigned seen[COLS * BM / 32];
+        int tn[TILES], rp[BM + 1];
+        Segments sg;
+    };
+    static constexpr int SMEM = WARPS * (int)((sizeof(Warp) + 15) / 16 * 16);
+};
+
+// A warp per panel of up to SMALL_N entries and COLS columns: its tiles are built in shared memory and written once, 16
+// bytes a lane, so the tile array needs no clearing and sees no scattered stores.  Longer panels become slices.
+template <typename V, int CLS>
+__global__ void __launch_bounds__(128) k_fill_small(int nb8, int rowA, const int *__restrict__ rowptr, const int *__restrict__ colidx, const V *__restrict__ val,
+                                                    const int *__restrict__ ucols, const int *__restrict__ ulen, ClassView v, V *__restrict__ tiles, ConvStats *st)
+{
+    using F = SmallFill<V, CLS>;
+    constexpr int PREC = F::PREC, BM = F::BM, BN = F::BN;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    typename F::Warp &w = *reinterpret_cast<typename F::Warp *>(smem_raw + warp * (F::SMEM / F::WARPS));
+    const int nnz0 = v.nnz_ptr[0];
+    for (int p = blockIdx.x * F::WARPS + warp; p < v.tilem; p += gridDim.x * F::WARPS)
+    {
+        const int row0 = v.panel_row[p], t0 = v.tile_ptr[p], nt = v.tile_ptr[p + 1] - t0;
+        if (nt == 0) continue;
+        __syncwarp();
+        if (lane <= BM) w.rp[lane] = rowptr[row0 + min(lane, rowA - row0)];
+        __syncwarp();
+        const int begin = w.rp[0], n = w.rp[BM] - begin;
+        if (!small_panel(PREC, CLS, n, nt))
         {
-            const int j = base + lane;
-            const bool active = j < je;
-            unsigned long long pos = ~0ull - (unsigned long long)lane;  // never equal between lanes
-            V v = V(0.0f);
-            if (active)
-            {
-                const int rank = lower_bound_dev(pcols + g0, d, colidx[j]);
-                const int t = rank / bn, c = rank - t * bn;
-                atomicAdd(&tn[t0 + t], 1);
-                if (k == 0)
+            if (CLS == 2 && lane == 0) push_slices(v, PREC, p, nt, st);   // 16-row panels: k_panel_lists did
+            continue;
+        }
+        int d;
+        if (CLS == 2)
+        {
+            d = ulen[row0 / 8];
+            for (int i = lane; i < d; i += 32) w.list[i] = ucols[begin + i];
+        }
+        else
+        {
+            const int keys = load_segments(w.sg, row0, 1, nb8, rowptr, ulen, lane);
+            d = warp_list(keys, lane, [&](int e) { return ucols[w.sg.find(e)]; }, [&](int pos, int c) { w.list[pos] = c; });
+        }
+        const int cols = nt * BN;
+        for (int i = lane; i < nt * (int)(BM * BN * sizeof(V) / 16); i += 32) reinterpret_cast<uint4 *>(w.image)[i] = make_uint4(0u, 0u, 0u, 0u);
+        for (int i = lane; i < (cols * BM + 31) / 32; i += 32) w.seen[i] = 0u;
+        for (int i = lane; i < nt; i += 32) w.tn[i] = 0;
+        __syncwarp();
+        const int last = w.list[d - 1];
+        for (int i = d + lane; i < cols; i += 32) w.list[i] = last;   // src/csr2tile.h:117-132
+        __syncwarp();
+        for (int i = lane; i < cols; i += 32) v.tile_colidx[(size_t)t0 * BN + i] = w.list[i];
+        bool twice = false;
+        for (int e = lane; e < n; e += 32)
+        {
+            const int j = begin + e, r = row_of<BM>(w.rp, j), rank = lower_bound_dev(w.list, d, colidx[j]), t = rank / BN;
+            const unsigned bit = (unsigned)(rank * BM + r), m = 1u << (bit & 31);
+            twice |= (atomicOr(&w.seen[bit >> 5], m) & m) != 0u;
+            atomicAdd(&w.tn[t], 1);
+            w.image[t * BM * BN + tsp_upstream_index(PREC, CLS, r, rank % BN)] = val[j];
+        }
+        if (__any_sync(0xffffffffu, twice))   // repeated entries: once more, row by row, adding in CSR order
+        {
+            __syncwarp();
+            for (int i = lane; i < nt * (int)(BM * BN * sizeof(V) / 16); i += 32) reinterpret_cast<uint4 *>(w.image)[i] = make_uint4(0u, 0u, 0u, 0u);
+            __syncwarp();
+            for (int r = 0; r < BM; r++)
+                for (int base = w.rp[r]; base < w.rp[r + 1]; base += 32)
                 {
-                    // row mask of (tile, row): 16-bit masks (TF32) are addressed as halves of 32-bit words
-                    const size_t bit = ((size_t)(t0 + t) * 64 + ri) * bn + c;
-                    atomicOr(&mask64[bit >> 5], 1u << (bit & 31));
+                    const int j = base + lane;
+                    const bool on = j < w.rp[r + 1];
+                    unsigned long long pos = ~0ull - (unsigned long long)lane;   // never equal between lanes
+                    V x = V(0.0f);
+                    if (on)
+                    {
+                        const int rank = lower_bound_dev(w.list, d, colidx[j]);
+                        pos = (unsigned long long)(rank / BN * BM * BN + tsp_upstream_index(PREC, CLS, r, rank % BN));
+                        x = val[j];
+                    }
+                    add_in_csr_order<V>(w.image, pos, x, on, lane);
                 }
-                else
-                {
-                    pos = (unsigned long long)(t0 + t) * (unsigned long long)(bm * bn) + (unsigned long long)tsp_upstream_index(precision, k, ri, c);
-                    v = val[j];
-                }
-            }
-            if (k != 0) add_in_csr_order<V>(vals, pos, v, active, lane);
+        }
+        __syncwarp();
+        uint4 *dst = reinterpret_cast<uint4 *>(tiles + (size_t)t0 * BM * BN);
+        for (int i = lane; i < nt * (int)(BM * BN * sizeof(V) / 16); i += 32) dst[i] = reinterpret_cast<const uint4 *>(w.image)[i];
+        int before = v.nnz_ptr[p] - nnz0;   // tile_nnz is the exclusive prefix of the entries per tile (src/csr2tile.h:786)
+        for (int i = 0; i < nt; i += 32)
+        {
+            const int c = i + lane < nt ? w.tn[i + lane] : 0;
+            int incl = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += y; }
+            if (i + lane < nt) v.tile_nnz[t0 + i + lane] = before + incl - c;
+            before += __shfl_sync(0xffffffffu, incl, 31);
         }
     }
 }
 
-// ---- stage 6: packed records of the 64-row class
-
-// One warp per tile: entries of the tile from its masks -> record size in 16-byte units (dense 4 KB record above
-// TSP_REC_MAX_VALS values), the dense flag, and the number of values before every row (row_off, 64 per tile).
-__global__ void k_rec_sizes(int tilenum, int precision, const unsigned int *__restrict__ mask64, unsigned int *__restrict__ units,
-                            unsigned char *__restrict__ dense, unsigned short *__restrict__ row_off)
+// exclusive prefix over a slice's per-tile counts -> tile_nnz; 256 threads
+__device__ __forceinline__ void write_tile_nnz(const int *tn, int nt, int before, int *dst)
 {
-    const int lane = threadIdx.x & 31;
-    const int warps = (gridDim.x * blockDim.x) >> 5;
-    const int vsz = precision ? 4 : 2, max_vals = TSP_REC_MAX_VALS(precision);
-    for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < tilenum; t += warps)
+    if (threadIdx.x >= 32) return;
+    const int lane = threadIdx.x;
+    for (int i = 0; i < nt; i += 32)
     {
-        // lane l owns rows 2l and 2l+1
-        unsigned int w0, w1;
-        if (precision) { const unsigned int w = mask64[(size_t)t * 32 + lane]; w0 = w & 0xffffu; w1 = w >> 16; }
-        else { w0 = mask64[(size_t)t * 64 + 2 * lane]; w1 = mask64[(size_t)t * 64 + 2 * lane + 1]; }
-        const int c0 = __popc(w0), cnt = c0 + __popc(w1);
-        int incl = cnt;
+        const int c = i + lane < nt ? tn[i + lane] : 0;
+        int incl = c;
+#pragma unroll
         for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += y; }
-        const int total = __shfl_sync(0xffffffffu, incl, 31);
-        row_off[(size_t)t * 64 + 2 * lane] = (unsigned short)(incl - cnt);
-        row_off[(size_t)t * 64 + 2 * lane + 1] = (unsigned short)(incl - cnt + c0);
-        if (lane == 0)
-        {
-            const bool is_dense = total > max_vals;
-            dense[t] = is_dense ? 1 : 0;
-            units[t] = is_dense ? (64u * tsp_bn(precision, 0) * vsz) / 16u : tsp_packed_units(precision, total);
-        }
+        if (i + lane < nt) dst[i + lane] = before + incl - c;
+        before += __shfl_sync(0xffffffffu, incl, 31);
     }
 }
 
-// rec[t] = exclusive prefix of the record sizes with the dense flag in bit 31; rec[tilenum] = total; units[] holds the
-// exclusive prefix on entry.
+// Slices of long 16- and 8-row panels, a CTA each: it reads all entries of the panel and keeps those of its columns.
+template <typename V, int CLS>
+__global__ void __launch_bounds__(256) k_fill_slices(int rowA, const int *__restrict__ rowptr, const int *__restrict__ colidx, const V *__restrict__ val,
+                                                     const int *__restrict__ ucols, const int *__restrict__ ulen, ClassView v, V *__restrict__ tiles, const ConvStats *st)
+{
+    constexpr int PREC = sizeof(V) == 4 ? 1 : 0, BM = CLS == 1 ? 16 : 8, BN = PREC ? 8 : 16, PER = SLICE_COLS / BN;
+    __shared__ int list[SLICE_COLS], tn[PER], rp[BM + 1], s_before, s_twice;
+    __shared__ unsigned seen[SLICE_COLS * BM / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, count = min(st->n_items[CLS], v.item_cap), nnz0 = v.nnz_ptr[0];
+    for (int w = blockIdx.x; w < count; w += gridDim.x)
+    {
+        __syncthreads();
+        const int p = v.items[w].x, s = v.items[w].y, row0 = v.panel_row[p];
+        const int t0 = v.tile_ptr[p] + s * PER, nt = min(v.tile_ptr[p + 1] - t0, PER), cols = nt * BN;
+        if (tid <= BM) rp[tid] = rowptr[row0 + min(tid, rowA - row0)];
+        if (tid == 0) { s_before = 0; s_twice = 0; }
+        for (int i = tid; i < nt; i += 256) tn[i] = 0;
+        for (int i = tid; i < (cols * BM + 31) / 32; i += 256) seen[i] = 0u;
+        uint4 *z = reinterpret_cast<uint4 *>(tiles + (size_t)t0 * BM * BN);
+        const int z16 = nt * (int)(BM * BN * sizeof(V) / 16);
+        for (int i = tid; i < z16; i += 256) z[i] = make_uint4(0u, 0u, 0u, 0u);
+        int *ci = v.tile_colidx + (size_t)t0 * BN;
+        if (CLS == 2)
+        {
+            const int d = ulen[row0 / 8] - s * SLICE_COLS;
+            const int *src = ucols + rowptr[row0] + s * SLICE_COLS;
+            for (int i = tid; i < cols; i += 256) { const int c = src[min(i, d - 1)]; list[i] = c; ci[i] = c; }   // padded with the last column
+        }
+        else for (int i = tid; i < cols; i += 256) list[i] = ci[i];
+        __syncthreads();
+        const int lo = list[0], hi = list[cols - 1];
+        int before = 0;
+        bool twice = false;
+#pragma unroll 2
+        for (int j = rp[0] + tid; j < rp[BM]; j += 256)
+        {
+            const int c = colidx[j];
+            before += c < lo;
+            if (c < lo || c > hi) continue;
+            const int r = row_of<BM>(rp, j), rank = lower_bound_dev(list, cols, c), t = rank / BN;
+            const unsigned bit = (unsigned)(rank * BM + r), m = 1u << (bit & 31);
+            twice |= (atomicOr(&seen[bit >> 5], m) & m) != 0u;
+            atomicAdd(&tn[t], 1);
+            tiles[(size_t)(t0 + t) * (BM * BN) + tsp_upstream_index(PREC, CLS, r, rank % BN)] = val[j];
+        }
+        for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+        if (lane == 0 && before) atomicAdd(&s_before, before);
+        if (twice) s_twice = 1;
+        __syncthreads();
+        if (s_twice)
+        {
+            for (int i = tid; i < z16; i += 256) z[i] = make_uint4(0u, 0u, 0u, 0u);
+            __syncthreads();
+            for (int r = warp; r < BM; r += 8)
+                for (int base = rp[r]; base < rp[r + 1]; base += 32)
+                {
+                    const int j = base + lane, c = j < rp[r + 1] ? colidx[j] : -1;
+                    const bool on = c >= lo && c <= hi;
+                    unsigned long long pos = ~0ull - (unsigned long long)lane;
+                    V x = V(0.0f);
+                    if (on)
+                    {
+                        const int rank = lower_bound_dev(list, cols, c);
+                        pos = (unsigned long long)(t0 + rank / BN) * (BM * BN) + (unsigned long long)tsp_upstream_index(PREC, CLS, r, rank % BN);
+                        x = val[j];
+                    }
+                    add_in_csr_order<V>(tiles, pos, x, on, lane);
+                }
+        }
+        write_tile_nnz(tn, nt, v.nnz_ptr[p] - nnz0 + s_before, v.tile_nnz + t0);
+    }
+}
+
+// ---- step 7: masks and packed records of the 64-row class
+
+template <int PREC>
+struct Masks64
+{
+    static constexpr int BN = PREC ? 16 : 32, PER = SLICE_COLS / BN;
+    struct Shared
+    {
+        unsigned masks[PER * 64 * BN / 32];
+        int list[SLICE_COLS], tn[PER], rp[65], before, twice;
+    };
+};
+
+// A CTA per slice of a 64-row panel: row masks of its tiles in shared memory -> global, entries per tile, and from the
+// masks the record size in 16-byte units (dense 4 KB record above TSP_REC_MAX_VALS values), the dense flag and the number
+// of values before every row (row_off, 64 per tile).  repeated[p] is set when the panel holds a (row, col) pair twice.
+template <int PREC>
+__global__ void __launch_bounds__(256) k_masks64(int rowA, const int *__restrict__ rowptr, const int *__restrict__ colidx, ClassView v, unsigned *__restrict__ mask64,
+                                                 unsigned *__restrict__ units, unsigned char *__restrict__ dense, unsigned short *__restrict__ row_off,
+                                                 unsigned char *__restrict__ repeated, const ConvStats *st)
+{
+    using M = Masks64<PREC>;
+    constexpr int BN = M::BN, PER = M::PER, TW = 64 * BN / 32;   // mask words of a tile
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    typename M::Shared &m = *reinterpret_cast<typename M::Shared *>(smem_raw);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, count = min(st->n_items[0], v.item_cap), nnz0 = v.nnz_ptr[0];
+    for (int w = blockIdx.x; w < count; w += gridDim.x)
+    {
+        __syncthreads();
+        const int p = v.items[w].x, s = v.items[w].y, row0 = v.panel_row[p];
+        const int t0 = v.tile_ptr[p] + s * PER, nt = min(v.tile_ptr[p + 1] - t0, PER), cols = nt * BN;
+        if (tid <= 64) m.rp[tid] = rowptr[row0 + min(tid, rowA - row0)];
+        if (tid == 0) { m.before = 0; m.twice = 0; }
+        for (int i = tid; i < nt; i += 256) m.tn[i] = 0;
+        for (int i = tid; i < nt * TW; i += 256) m.masks[i] = 0u;
+        for (int i = tid; i < cols; i += 256) m.list[i] = v.tile_colidx[(size_t)t0 * BN + i];
+        __syncthreads();
+        const int lo = m.list[0], hi = m.list[cols - 1];
+        int before = 0;
+        bool twice = false;
+#pragma unroll 2
+        for (int j = m.rp[0] + tid; j < m.rp[64]; j += 256)
+        {
+            const int c = colidx[j];
+            before += c < lo;
+            if (c < lo || c > hi) continue;
+            const int r = row_of<64>(m.rp, j), rank = lower_bound_dev(m.list, cols, c), t = rank / BN;
+            const unsigned bit = (unsigned)((t * 64 + r) * BN + rank % BN), b = 1u << (bit & 31);
+            twice |= (atomicOr(&m.masks[bit >> 5], b) & b) != 0u;
+            atomicAdd(&m.tn[t], 1);
+        }
+        for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+        if (lane == 0 && before) atomicAdd(&m.before, before);
+        if (twice) m.twice = 1;
+        __syncthreads();
+        if (tid == 0 && m.twice) repeated[p] = 1;
+        for (int i = tid; i < nt * TW; i += 256) mask64[(size_t)t0 * TW + i] = m.masks[i];
+        for (int t = warp; t < nt; t += 8)
+        {
+            unsigned w0, w1;   // lane l owns rows 2l and 2l+1
+            if (PREC) { const unsigned x = m.masks[t * TW + lane]; w0 = x & 0xffffu; w1 = x >> 16; }
+            else { w0 = m.masks[t * TW + 2 * lane]; w1 = m.masks[t * TW + 2 * lane + 1]; }
+            const int c0 = __popc(w0), cnt = c0 + __popc(w1);
+            int incl = cnt;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += y; }
+            const int total = __shfl_sync(0xffffffffu, incl, 31);
+            reinterpret_cast<unsigned *>(row_off)[(size_t)(t0 + t) * 32 + lane] = (unsigned)(incl - cnt) | (unsigned)(incl - cnt + c0) << 16;
+            if (lane == 0)
+            {
+                const bool is_dense = total > TSP_REC_MAX_VALS(PREC);
+                dense[t0 + t] = is_dense ? 1 : 0;
+                units[t0 + t] = is_dense ? 4096u / 16u : tsp_packed_units(PREC, total);
+            }
+        }
+        write_tile_nnz(m.tn, nt, v.nnz_ptr[p] - nnz0 + m.before, v.tile_nnz + t0);
+    }
+}
+
+// rec[t] = exclusive prefix of the record sizes with the dense flag in bit 31; rec[tilenum] = total
 __global__ void k_rec_finish(int tilenum, const unsigned int *__restrict__ prefix, const unsigned char *__restrict__ dense,
                              unsigned int *__restrict__ rec)
 {
@@ -641,56 +1244,58 @@ __global__ void k_init_positions(int tilenum, int precision, const unsigned int 
     }
 }
 
-// One warp per original row of the 64-row class: every entry's value goes to its place in the tile's record -- for a
-// packed record the slot given by the masks (row-major order of the set bits), together with the entry's position in
-// the operand tile; for a dense record the operand position itself.
+// Every entry of the 64-row class goes to its place in its tile's record -- for a packed record the slot given by the
+// masks (row-major order of the set bits), together with the entry's position in the operand tile; for a dense record the
+// operand position itself.  A CTA per chunk of CHUNK_N entries; a panel with repeated entries is one CTA's work, a warp
+// per row, adding in CSR order.
 template <typename V>
-__global__ void k_place_values64(int rowA, int precision, int s0, int s1, const int *__restrict__ rowptr, const int *__restrict__ colidx,
-                                 const V *__restrict__ val, const int *__restrict__ blk_seq, const unsigned char *__restrict__ seq_cls,
-                                 const int *__restrict__ seq_idx, const int *__restrict__ seq_blk, const int *__restrict__ pptr,
-                                 const int *__restrict__ pcols, int p0_64, const int *__restrict__ tp64, const unsigned int *__restrict__ mask64,
-                                 const unsigned short *__restrict__ row_off, const unsigned int *__restrict__ rec, V *pack)
+__global__ void __launch_bounds__(256) k_place_values64(int rowA, const int *__restrict__ rowptr, const int *__restrict__ colidx, const V *__restrict__ val,
+                                                        ClassView v, const int2 *__restrict__ chunks, int chunk_cap, const unsigned int *__restrict__ mask64,
+                                                        const unsigned short *__restrict__ row_off, const unsigned int *__restrict__ rec,
+                                                        const unsigned char *__restrict__ repeated, V *pack, const ConvStats *st)
 {
-    const int lane = threadIdx.x & 31;
-    const int warps = (gridDim.x * blockDim.x) >> 5;
-    const int bn = tsp_bn(precision, 0), per16 = 16 / (int)sizeof(V), per = 2 + (int)sizeof(V);
-    for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rowA; r += warps)
+    constexpr int PREC = sizeof(V) == 4 ? 1 : 0, BN = PREC ? 16 : 32, PER16 = 16 / (int)sizeof(V), PER = 2 + (int)sizeof(V);
+    __shared__ int rp[65];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, count = min(st->n_chunks, chunk_cap);
+    for (int w = blockIdx.x; w < count; w += gridDim.x)
     {
-        const int s = blk_seq[r >> 3];
-        if (s < s0 || s >= s1 || seq_cls[s] != 0) continue;
-        const int jb = rowptr[r], je = rowptr[r + 1];
-        if (jb == je) continue;
-        const int t0 = tp64[seq_idx[s] - p0_64];
-        const int ri = r - seq_blk[s] * 8;
-        const int g0 = pptr[s], d = pptr[s + 1] - g0;
-        for (int base = jb; base < je; base += 32)
+        __syncthreads();
+        const int p = chunks[w].x, s = chunks[w].y, row0 = v.panel_row[p], t0 = v.tile_ptr[p], nt = v.tile_ptr[p + 1] - t0;
+        const int *list = v.tile_colidx + (size_t)t0 * BN;   // its tail repeats the last column, which changes no rank
+        const bool ordered = repeated[p] != 0;
+        if (ordered && s > 0) continue;
+        if (tid <= 64) rp[tid] = rowptr[row0 + min(tid, rowA - row0)];
+        __syncthreads();
+        auto place = [&](int j, int r) {   // position of entry j in `pack`, counted in values; writes the position slot
+            const int rank = lower_bound_dev(list, nt * BN, colidx[j]), t = t0 + rank / BN, c = rank % BN;
+            const unsigned int rw = rec[t];
+            const unsigned long long rec_elem = (unsigned long long)(rw & 0x7fffffffu) * PER16;
+            if (rw >> 31) return rec_elem + (unsigned long long)tsp_umma_index(PREC, r, c);
+            const size_t bit = ((size_t)t * 64 + r) * BN;          // first bit of the row mask
+            unsigned int m = mask64[bit >> 5] >> (bit & 31);
+            if (PREC) m &= 0xffffu;
+            const unsigned int n_pad = ((rec[t + 1] & 0x7fffffffu) - rw) * 16u / PER;
+            const unsigned int slot = row_off[(size_t)t * 64 + r] + __popc(m & ((1u << c) - 1u));
+            // positions first (2 bytes each), then the values: n_pad * 2 bytes is a multiple of 16
+            reinterpret_cast<unsigned short *>(pack + (size_t)rw * PER16)[slot] = (unsigned short)tsp_umma_index(PREC, r, c);
+            return rec_elem + (unsigned long long)(n_pad * 2u / sizeof(V)) + slot;
+        };
+        if (!ordered)
         {
-            const int j = base + lane;
-            const bool active = j < je;
-            unsigned long long pos = ~0ull - (unsigned long long)lane;
-            V v = V(0.0f);
-            if (active)
-            {
-                const int rank = lower_bound_dev(pcols + g0, d, colidx[j]);
-                const int t = t0 + rank / bn, c = rank % bn;
-                const unsigned int rw = rec[t];
-                const unsigned long long rec_elem = (unsigned long long)(rw & 0x7fffffffu) * per16;
-                if (rw >> 31) pos = rec_elem + (unsigned long long)tsp_umma_index(precision, ri, c);
-                else
-                {
-                    const size_t bit = ((size_t)t * 64 + ri) * bn;          // first bit of the row mask
-                    unsigned int m = mask64[bit >> 5] >> (bit & 31);
-                    if (precision) m &= 0xffffu;
-                    const unsigned int n_pad = ((rec[t + 1] & 0x7fffffffu) - rw) * 16u / per;
-                    const unsigned int slot = row_off[(size_t)t * 64 + ri] + __popc(m & ((1u << c) - 1u));
-                    // positions first (2 bytes each), then the values: n_pad * 2 bytes is a multiple of 16
-                    pos = rec_elem + (unsigned long long)(n_pad * 2u / sizeof(V)) + slot;
-                    reinterpret_cast<unsigned short *>(pack + (size_t)rw * per16)[slot] = (unsigned short)tsp_umma_index(precision, ri, c);
-                }
-                v = val[j];
-            }
-            add_in_csr_order<V>(pack, pos, v, active, lane);
+            const int end = min(rp[0] + (s + 1) * CHUNK_N, rp[64]);
+            for (int j = rp[0] + s * CHUNK_N + tid; j < end; j += 256) pack[place(j, row_of<64>(rp, j))] = val[j];
+            continue;
         }
+        for (int r = warp; r < 64; r += 8)
+            for (int base = rp[r]; base < rp[r + 1]; base += 32)
+            {
+                const int j = base + lane;
+                const bool on = j < rp[r + 1];
+                unsigned long long pos = ~0ull - (unsigned long long)lane;
+                V x = V(0.0f);
+                if (on) { pos = place(j, r); x = val[j]; }
+                add_in_csr_order<V>(pack, pos, x, on, lane);
+            }
     }
 }
 
@@ -729,37 +1334,9 @@ __global__ void k_export64(int tilenum, int precision, const unsigned int *__res
     }
 }
 
+
 inline int blocks_for(long long n, int threads) { return (int)((n + threads - 1) / threads > 0 ? (n + threads - 1) / threads : 1); }
-
-// Radix sort on the bits in use, then unique.  keys/tmp are swapped so that the result is in `keys`; the number of
-// distinct keys is left in *d_count (device).
-int sort_unique_keys(unsigned long long *&keys, unsigned long long *&tmp, int n, int key_bits, void *scratch, size_t scratch_bytes,
-                     int *d_count)
-{
-    cub::DoubleBuffer<unsigned long long> db(keys, tmp);
-    size_t bytes = scratch_bytes;
-    TSP_CUDA(cub::DeviceRadixSort::SortKeys(scratch, bytes, db, n, 0, key_bits));
-    unsigned long long *sorted = db.Current(), *other = db.Alternate();
-    bytes = scratch_bytes;
-    TSP_CUDA(cub::DeviceSelect::Unique(scratch, bytes, sorted, other, d_count, n));
-    keys = other; tmp = sorted;
-    return TSP_OK;
-}
-
-size_t sort_unique_scratch_bytes(int n)
-{
-    size_t a = 0, b = 0;
-    cub::DoubleBuffer<unsigned long long> db(nullptr, nullptr);
-    cub::DeviceRadixSort::SortKeys(nullptr, a, db, n, 0, 64);
-    cub::DeviceSelect::Unique(nullptr, b, (unsigned long long *)nullptr, (unsigned long long *)nullptr, (int *)nullptr, n);
-    size_t c = 0, d = 0;   // the prefix sums over panels share the same scratch
-    cub::DeviceScan::ExclusiveSum(nullptr, c, (int *)nullptr, (int *)nullptr, n + 1);
-    cub::DeviceScan::InclusiveSum(nullptr, d, (double *)nullptr, (double *)nullptr, n + 1);
-    if (b > a) a = b;
-    if (c > a) a = c;
-    if (d > a) a = d;
-    return a + 256;
-}
+inline int capped(long long n, int most) { return (int)(n < 1 ? 1 : (n > most ? most : n)); }
 
 int bits_for(unsigned long long v)
 {
@@ -768,11 +1345,51 @@ int bits_for(unsigned long long v)
     return b;
 }
 
-// small pinned host buffer for scalar read-backs
-int pinned(tsp_handle *h, int **p)
+// shared words of the bitmap kernels: all columns when they fit 128 KB (2^20 columns), else several passes
+int bitmap_words(int colA)
 {
-    if (!h->h_pin) TSP_CUDA(cudaMallocHost(&h->h_pin, 4096));
-    *p = static_cast<int *>(h->h_pin);
+    const long long w = ((long long)colA + 32767) / 32768 * 1024;
+    return w > 32768 ? 32768 : (int)w;
+}
+
+// small pinned host buffer for read-backs
+int pinned(tsp_handle *h, ConvStats **p)
+{
+    if (!h->h_pin) TSP_CUDA(cudaMallocHost(&h->h_pin, sizeof(ConvStats) + 256));
+    *p = static_cast<ConvStats *>(h->h_pin);
+    return TSP_OK;
+}
+
+// kernels with more than 48 KB of dynamic shared memory; once per device
+int configure_kernels(int device)
+{
+    static bool done[64] = {false};
+    if (device < 64 && done[device]) return TSP_OK;
+    const int attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    TSP_CUDA(cudaFuncSetAttribute(k_block_lists_big, (cudaFuncAttribute)attr, 32768 * 4));
+    TSP_CUDA(cudaFuncSetAttribute(k_panel_lists_big, (cudaFuncAttribute)attr, 32768 * 4));
+    TSP_CUDA(cudaFuncSetAttribute(k_fill_small<__half, 1>, (cudaFuncAttribute)attr, SmallFill<__half, 1>::SMEM));
+    TSP_CUDA(cudaFuncSetAttribute(k_fill_small<__half, 2>, (cudaFuncAttribute)attr, SmallFill<__half, 2>::SMEM));
+    TSP_CUDA(cudaFuncSetAttribute(k_fill_small<float, 1>, (cudaFuncAttribute)attr, SmallFill<float, 1>::SMEM));
+    TSP_CUDA(cudaFuncSetAttribute(k_fill_small<float, 2>, (cudaFuncAttribute)attr, SmallFill<float, 2>::SMEM));
+    TSP_CUDA(cudaFuncSetAttribute(k_masks64<0>, (cudaFuncAttribute)attr, (int)sizeof(Masks64<0>::Shared)));
+    TSP_CUDA(cudaFuncSetAttribute(k_masks64<1>, (cudaFuncAttribute)attr, (int)sizeof(Masks64<1>::Shared)));
+    if (device < 64) done[device] = true;
+    return TSP_OK;
+}
+
+template <typename V, int CLS>
+int fill_class(tsp_handle *h, int nb8, const int *rowptr, const int *colidx, const V *val, const int *ucols, const int *ulen, const ClassView &v,
+               long long entries, ConvStats *d_stats, cudaStream_t st)
+{
+    using F = SmallFill<V, CLS>;
+    if (v.tilem == 0) return TSP_OK;
+    V *tiles = (V *)h->cls[CLS].d_val;
+    k_fill_small<V, CLS><<<capped((v.tilem + F::WARPS - 1) / F::WARPS, 148 * 32), 32 * F::WARPS, F::SMEM, st>>>(nb8, h->rowA, rowptr, colidx, val, ucols, ulen, v, tiles, d_stats);
+    // a panel is long when it has more than SMALL_N entries or more than small_cols() - BN columns, hence as many entries
+    if (entries > small_cols(F::PREC, CLS) - F::BN)
+        k_fill_slices<V, CLS><<<capped(v.item_cap, 148 * 8), 256, 0, st>>>(h->rowA, rowptr, colidx, val, ucols, ulen, v, tiles, d_stats);
+    TSP_CUDA(cudaGetLastError());
     return TSP_OK;
 }
 
@@ -813,7 +1430,7 @@ void tsp_free_tiles(tsp_handle *h, bool release)
 }
 
 // One allocation for every tile array of the three classes; sizes come from cls[k].tilem and cls[k].tilenum.
-// tile_ptr (inputs of a scan), tile_nnz (atomic counters), the dense values and the masks start as zeros.
+// Nothing is cleared: the conversion (or tsp_load) writes every element that anything reads.
 int tsp_alloc_tile_arrays(tsp_handle *h)
 {
     const size_t vsz = h->precision ? 4 : 2;
@@ -849,14 +1466,6 @@ int tsp_alloc_tile_arrays(tsp_handle *h)
         c.d_tile_colidx = (int *)(base + at[k][3]);
         if (k == 0) { c.d_bitmap = base + at[k][4]; c.d_rec = (unsigned int *)(base + at[k][5]); c.d_val = nullptr; }
         else c.d_val = base + at[k][4];
-    }
-    // zero: everything except the column indices (fully written later); cheaper as a few ranges than as one memset of all
-    for (int k = 0; k < 3; k++)
-    {
-        const size_t from = at[k][0], to = at[k][3];
-        TSP_CUDA(cudaMemsetAsync(base + from, 0, to - from, 0));
-        const size_t vend = k == 2 ? off : at[k + 1][0];
-        TSP_CUDA(cudaMemsetAsync(base + at[k][4], 0, vend - at[k][4], 0));
     }
     return TSP_OK;
 }
@@ -905,6 +1514,24 @@ int tsp_export_values_upstream(const tsp_handle *h, int cls, void *h_dst)
     return TSP_OK;
 }
 
+
+// Host copies of tile_ptr and the panel rows: only exports, the tile cache and matrices with very long panels need them, so
+// they are fetched on first use instead of on every conversion.
+int tsp_fetch_panels(const tsp_handle *h, int cls)
+{
+    static std::mutex mutex;   // two threads may export from one handle
+    std::lock_guard<std::mutex> lock(mutex);
+    const TspClass &c = h->cls[cls];
+    if (c.h_tile_ptr.size() == (size_t)c.tilem + 1) return TSP_OK;
+    std::vector<int> tp((size_t)c.tilem + 1), pr((size_t)c.tilem);
+    TSP_CUDA(cudaSetDevice(h->device));
+    TSP_CUDA(cudaMemcpy(tp.data(), c.d_tile_ptr, tp.size() * 4, cudaMemcpyDeviceToHost));
+    if (c.tilem) TSP_CUDA(cudaMemcpy(pr.data(), c.d_panel_row, pr.size() * 4, cudaMemcpyDeviceToHost));
+    c.h_panel_row.swap(pr);
+    c.h_tile_ptr.swap(tp);
+    return TSP_OK;
+}
+
 int tsp_convert_impl(tsp_handle *h, int rowA, int colA, long long nnz64, const int *rowptr_in, const int *colidx_in,
                      const void *val_in, bool csr_on_host, float gamma, float delta, int shard_index, int shard_count)
 {
@@ -919,12 +1546,13 @@ int tsp_convert_impl(tsp_handle *h, int rowA, int colA, long long nnz64, const i
     h->rowA = rowA; h->colA = colA; h->nnzA = nnz64;
     const int nnz = (int)nnz64;
     const int prec = h->precision;
-    const int nb8 = (rowA + 7) / 8;
+    const int nb8 = rowA / 8 + (rowA % 8 != 0);
     const int T = 256;
     const int nchunk = (nb8 + CHAIN_L - 1) / CHAIN_L;
     cudaStream_t st = 0;
-    int *pin = nullptr;
+    ConvStats *pin = nullptr;
     TSP_TRY(pinned(h, &pin));
+    TSP_TRY(configure_kernels(h->device));
 
     // TSP_CONVERT_TRACE=1: wall time of every phase on stderr (each mark waits for the stream, so the total grows a little)
     static const bool trace = getenv("TSP_CONVERT_TRACE") != nullptr;
@@ -943,14 +1571,14 @@ int tsp_convert_impl(tsp_handle *h, int rowA, int colA, long long nnz64, const i
     if (gamma <= 0.0f) fixed = 0;
     else if (gamma >= 4.0f && delta <= 0.0f) fixed = 1;
     else if (gamma >= 4.0f && delta > 2.0f) fixed = 2;
-    const bool want64 = fixed < 0 && gamma < 4.0f;
-    const bool want16 = fixed < 0 && (want64 || (delta > 0.0f && !(delta > 2.0f)));
+    // how many blocks back a column has to be looked for: 7 where 64-row windows count, 1 for 16-row windows alone
+    const int reach = fixed == 0 || (fixed < 0 && gamma < 4.0f) ? 7 : (fixed == 2 ? 0 : 1);
 
     // ---- workspace: everything whose size follows from nnz and rowA, in one chunk
-    const size_t cub_bytes = sort_unique_scratch_bytes(nnz > nb8 + 2 ? nnz : nb8 + 2);
     {
         const size_t n = (size_t)(nnz ? nnz : 1), b = (size_t)nb8 + 16;
-        size_t need = 3 * n * 8 + 2 * n * 4 + b * (4 * 9 + 3) + (size_t)nchunk * (8 + 96 + 4 + 12) + b * 8 + cub_bytes + 64 * 256 + (1 << 16);
+        size_t need = n * 4 + b * (4 + 32 + 4 * 2 + 1 + 4 + 9 * 4) + (size_t)nchunk * (8 + 8 * 4 * CHAIN_N + 4 + 4 * CHAIN_N) + sizeof(ConvStats) + 64 * 256 + (1 << 16);
+        if (shard_count > 1) need += b * (4 * 3 + 1 + 8);
         if (csr_on_host) need += ((size_t)rowA + 1) * 4 + n * (4 + (prec ? 4 : 2)) + 1024;
         TSP_TRY(reserve_workspace(h, need));
     }
@@ -972,7 +1600,7 @@ int tsp_convert_impl(tsp_handle *h, int rowA, int colA, long long nnz64, const i
         TSP_CUDA(cudaMemcpyAsync(rp, rowptr_in, ((size_t)rowA + 1) * 4, cudaMemcpyHostToDevice, st));
         if (nnz) TSP_CUDA(cudaMemcpyAsync(ci, colidx_in, (size_t)nnz * 4, cudaMemcpyHostToDevice, st));
         d_rowptr = rp; d_colidx = ci; d_val = vv;
-        values_pending = nnz > 0;   // the values are not needed before stage 5: their upload overlaps the partition kernels
+        values_pending = nnz > 0;   // the values are not needed before step 6: their upload overlaps the partition kernels
     }
     auto upload_values = [&]() -> int {
         if (!values_pending || values_in_flight) return TSP_OK;
@@ -986,273 +1614,213 @@ int tsp_convert_impl(tsp_handle *h, int rowA, int colA, long long nnz64, const i
         values_in_flight = false;
         return TSP_OK;
     };
-    unsigned long long *keys, *keys_tmp, *keys_col = nullptr, *class_rows_nnz;
-    int *u8_ptr, *ucols, *n16, *n64, *entry, *base, *counts, *seq_blk, *seq_idx, *blk_seq, *scalars, *pptr_buf, *pcols_buf, *seq_tiles;
-    unsigned char *cls_of, *exit_off, *seq_cls, *cub_tmp;
-    double *cost;
-    TSP_TRY(ws.get(&keys, nnz)); TSP_TRY(ws.get(&keys_tmp, nnz)); TSP_TRY(ws.get(&u8_ptr, (size_t)nb8 + 9)); TSP_TRY(ws.get(&ucols, nnz));
-    TSP_TRY(ws.get(&n16, (size_t)nb8 + 2)); TSP_TRY(ws.get(&n64, (size_t)nb8 + 2)); TSP_TRY(ws.get(&cls_of, nb8));
-    TSP_TRY(ws.get(&exit_off, (size_t)nchunk * 8)); TSP_TRY(ws.get(&counts, (size_t)nchunk * 24)); TSP_TRY(ws.get(&entry, nchunk));
-    TSP_TRY(ws.get(&base, (size_t)nchunk * 3 + 3));
-    TSP_TRY(ws.get(&seq_blk, nb8)); TSP_TRY(ws.get(&seq_cls, nb8)); TSP_TRY(ws.get(&seq_idx, nb8)); TSP_TRY(ws.get(&blk_seq, nb8));
-    TSP_TRY(ws.get(&class_rows_nnz, 6)); TSP_TRY(ws.get(&scalars, 64)); TSP_TRY(ws.get(&cub_tmp, cub_bytes));
-    TSP_TRY(ws.get(&pptr_buf, (size_t)nb8 + 1)); TSP_TRY(ws.get(&pcols_buf, nnz)); TSP_TRY(ws.get(&seq_tiles, nb8));
-    TSP_TRY(ws.get(&cost, nb8));
-    if (want16 || want64) TSP_TRY(ws.get(&keys_col, nnz));
-    // scalars: [0] distinct (8-row block, column) pairs, [1] CSR check, [2] distinct (panel, column) pairs, [8..17] shard cuts
-    int *d_nu = scalars, *d_bad = scalars + 1, *d_np = scalars + 2, *d_cuts = scalars + 8;
-    TSP_CUDA(cudaMemsetAsync(scalars, 0, 64 * sizeof(int), st));
-    TSP_CUDA(cudaMemsetAsync(class_rows_nnz, 0, 6 * sizeof(unsigned long long), st));
+    ConvStats *d_stats;
+    int *ucols, *ulen, *fresh = nullptr, *mid, *big, *tiles_of, *entry, *base, *counts;
+    unsigned char *cls_of, *exit_off;
+    ClassArrays all;
+    SeqArrays seq = {nullptr, nullptr, nullptr, nullptr};
+    TSP_TRY(ws.get(&d_stats, 1)); TSP_TRY(ws.get(&ucols, nnz)); TSP_TRY(ws.get(&ulen, (size_t)nb8 + 16));
+    TSP_TRY(ws.get(&mid, nb8)); TSP_TRY(ws.get(&big, nb8));
+    if (reach) TSP_TRY(ws.get(&fresh, ((size_t)nb8 + 8) * 8));
+    TSP_TRY(ws.get(&cls_of, nb8)); TSP_TRY(ws.get(&tiles_of, nb8));
+    TSP_TRY(ws.get(&exit_off, (size_t)nchunk * 8)); TSP_TRY(ws.get(&counts, (size_t)nchunk * 8 * CHAIN_N)); TSP_TRY(ws.get(&entry, nchunk));
+    TSP_TRY(ws.get(&base, (size_t)nchunk * CHAIN_N));
+    for (int k = 0; k < 3; k++) { TSP_TRY(ws.get(&all.tile_ptr[k], (size_t)nb8 + 1)); TSP_TRY(ws.get(&all.nnz_ptr[k], (size_t)nb8 + 1)); TSP_TRY(ws.get(&all.panel_row[k], nb8)); }
+    if (shard_count > 1) { TSP_TRY(ws.get(&seq.blk, nb8)); TSP_TRY(ws.get(&seq.idx, nb8)); TSP_TRY(ws.get(&seq.tiles, nb8)); TSP_TRY(ws.get(&seq.cls, nb8)); }
+    TSP_CUDA(cudaMemsetAsync(d_stats, 0, sizeof(ConvStats), st));
 
     mark("workspace + upload");
-    // ---- stage 1: sorted distinct columns of every 8-row block
-    nvtxRangePushA("tsp convert: partition (stages 1-3)");
+    // ---- steps 1 - 3
+    const int bits = bits_for((unsigned long long)colA), words = bitmap_words(colA);
     {
-        const int blocks = blocks_for((long long)rowA * 32, T) > 148 * 64 ? 148 * 64 : blocks_for((long long)rowA * 32, T);
-        k_make_block_keys<<<blocks, T, 0, st>>>(rowA, colA, nnz, d_rowptr, d_colidx, keys, d_bad);   // also checks the row pointers of an empty matrix
+        TspRange range("tsp convert: partition (steps 1-3)");
+        k_block_lists<<<capped((nb8 + 16 + 7) / 8, 148 * 64), T, 0, st>>>(nb8, rowA, colA, nnz, d_rowptr, d_colidx, ucols, ulen, mid, big, d_stats);
+        if (nnz > SMALL_N) k_block_lists_mid<<<capped(nnz / SMALL_N, 148 * 5), T, 0, st>>>(rowA, colA, nnz, bits, d_rowptr, d_colidx, ucols, ulen, mid, d_stats);
+        if (nnz > MID_N) k_block_lists_big<<<capped(nnz / MID_N, 148), 1024, words * 4, st>>>(rowA, colA, nnz, words, d_rowptr, d_colidx, ucols, ulen, big, d_stats);
         TSP_CUDA(cudaGetLastError());
-        if (nnz > 0) TSP_TRY(sort_unique_keys(keys, keys_tmp, nnz, 32 + bits_for((unsigned long long)nb8), cub_tmp, cub_bytes, d_nu));
-    }
-    {
-        // the values go up on a side stream while the partition kernels run
-        const int rc_up = upload_values();
-        if (rc_up != TSP_OK) { nvtxRangePop(); return rc_up; }
-    }
-    mark("stage 1 keys+sort+unique");
-    k_group_offsets<<<blocks_for(nb8 + 9, T), T, 0, st>>>(keys, d_nu, nb8, 8, u8_ptr);   // windows near the end index past nb8
-    if (nnz > 0) k_low_words<<<blocks_for(nnz, T) > 148 * 16 ? 148 * 16 : blocks_for(nnz, T), T, 0, st>>>(keys, d_nu, ucols);
-    TSP_CUDA(cudaGetLastError());
-
-    // ---- stage 2 + 3: window counts, decisions, chain
-    if (want16 || want64)
-    {
-        // read-back 0 (only when windows are compared at all): the number of pairs, and the CSR check
-        TSP_CUDA(cudaMemcpyAsync(pin, scalars, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
-        TSP_CUDA(cudaStreamSynchronize(st));
-        if (pin[1])
+        TSP_TRY(upload_values());   // the values go up on a side stream while the partition kernels run
+        mark("step 1 block lists");
+        if (reach)
         {
-            nvtxRangePop();
-            tsp_set_error("convert: the CSR is inconsistent (row pointers must start at 0, not decrease and end at nnz; columns must lie in [0, %d))", colA);
-            return TSP_EINVAL;
-        }
-        const int pairs = pin[0], bb = bits_for((unsigned long long)nb8);
-        TSP_CUDA(cudaMemsetAsync(n16, 0, ((size_t)nb8 + 2) * 4, st)); TSP_CUDA(cudaMemsetAsync(n64, 0, ((size_t)nb8 + 2) * 4, st));
-        if (pairs > 0)
-        {
-            k_col_block_keys<<<blocks_for(pairs, T), T, 0, st>>>(keys, pairs, bb, keys_tmp);
-            cub::DoubleBuffer<unsigned long long> db(keys_tmp, keys_col);
-            size_t bytes = cub_bytes;
-            TSP_CUDA(cub::DeviceRadixSort::SortKeys(cub_tmp, bytes, db, pairs, 0, bb + bits_for((unsigned long long)colA), st));
-            k_window_diffs<<<blocks_for(pairs, T), T, 0, st>>>(db.Current(), pairs, bb, want64 ? 1 : 0, n16, n64);
+            const int warp_ctas = capped((nb8 + 8 + 7) / 8, 148 * 32), list_ctas = nnz > SMALL_N ? capped(nnz / SMALL_N, 148 * 4) : 0;
+            k_fresh_columns<<<warp_ctas + list_ctas, T, 0, st>>>(nb8, rowA, nnz, reach, warp_ctas, d_rowptr, ucols, ulen, mid, big, d_stats, fresh);
             TSP_CUDA(cudaGetLastError());
-            bytes = cub_bytes;
-            TSP_CUDA(cub::DeviceScan::InclusiveSum(cub_tmp, bytes, n16, n16, nb8 + 1, st));
-            bytes = cub_bytes;
-            if (want64) TSP_CUDA(cub::DeviceScan::InclusiveSum(cub_tmp, bytes, n64, n64, nb8 + 1, st));
         }
+        mark("step 2 window counts");
+        k_chain_local<<<(nchunk + LOCAL_CHUNKS - 1) / LOCAL_CHUNKS, LOCAL_CHUNKS * 8, 0, st>>>(nb8, nchunk, rowA, nnz, prec, gamma, delta, fixed, reach, d_rowptr, ulen,
+                                                                                              fresh, cls_of, tiles_of, exit_off, counts);
+        k_chain_compose<<<1, 1024, 0, st>>>(nchunk, exit_off, counts, entry, base, d_stats);
+        k_chain_emit<<<(nchunk + EMIT_CHUNKS - 1) / EMIT_CHUNKS, 128, 0, st>>>(nb8, nchunk, rowA, nnz, cls_of, tiles_of, entry, base, d_rowptr, all, seq, d_stats);
+        TSP_CUDA(cudaGetLastError());
+        TSP_CUDA(cudaMemcpyAsync(pin, d_stats, sizeof(ConvStats), cudaMemcpyDeviceToHost, st));
+        TSP_CUDA(cudaStreamSynchronize(st));
     }
-    mark("stage 2 window counts");
-    k_decide<<<blocks_for(nb8, T), T, 0, st>>>(nb8, rowA, gamma, delta, fixed, u8_ptr, n16, n64, cls_of);
-    k_chain_local<<<blocks_for((long long)nchunk * 8, 256), 256, 0, st>>>(nb8, nchunk, cls_of, exit_off, counts);
-    k_chain_compose<<<1, 1024, 0, st>>>(nchunk, exit_off, counts, entry, base);
-    k_chain_emit<<<blocks_for(nchunk, 128), 128, 0, st>>>(nb8, nchunk, rowA, cls_of, entry, base, d_rowptr, seq_blk, seq_cls, seq_idx, blk_seq,
-                                                        class_rows_nnz);
-    TSP_CUDA(cudaGetLastError());
-    // read-back 1: distinct count, CSR check, panels per class, rows and entries per class
-    TSP_CUDA(cudaMemcpyAsync(pin, scalars, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
-    TSP_CUDA(cudaMemcpyAsync(pin + 2, base + (size_t)nchunk * 3, 3 * sizeof(int), cudaMemcpyDeviceToHost, st));
-    TSP_CUDA(cudaMemcpyAsync(pin + 8, class_rows_nnz, 6 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-    TSP_CUDA(cudaStreamSynchronize(st));
-    nvtxRangePop();
-    mark("stage 3 decide+chain+readback");
-    const int nu = pin[0];
-    if (pin[1])
+    mark("step 3 chain + readback");
+    if (pin->bad)
     {
         tsp_set_error("convert: the CSR is inconsistent (row pointers must start at 0, not decrease and end at nnz; columns must lie in [0, %d))", colA);
         return TSP_EINVAL;
     }
-    const int totals[3] = {pin[2], pin[3], pin[4]};
-    unsigned long long tot_rows_nnz[6];
-    memcpy(tot_rows_nnz, pin + 8, sizeof(tot_rows_nnz));
-    const int nseq = totals[0] + totals[1] + totals[2];
 
-    // ---- stage 4: sorted distinct columns of every panel
-    TspRange range_tiles("tsp convert: tiles (stages 4-6)");
-    const int *pptr = nullptr, *pcols = nullptr;
-    const bool all8 = totals[0] == 0 && totals[1] == 0;
-    if (all8) { pptr = u8_ptr; pcols = ucols; }  // an 8-row panel is one 8-row block
-    else
-    {
-        if (nu)
-        {
-            k_make_panel_keys<<<blocks_for(nu, T), T, 0, st>>>(keys, nu, blk_seq, keys_tmp);
-            TSP_CUDA(cudaGetLastError());
-            { unsigned long long *t = keys; keys = keys_tmp; keys_tmp = t; }
-            TSP_TRY(sort_unique_keys(keys, keys_tmp, nu, 32 + bits_for((unsigned long long)nseq), cub_tmp, cub_bytes, d_np));
-        }
-        k_group_offsets<<<blocks_for(nseq + 1, T), T, 0, st>>>(keys, d_np, nseq, 0, pptr_buf);
-        if (nu) k_low_words<<<blocks_for(nu, T) > 148 * 16 ? 148 * 16 : blocks_for(nu, T), T, 0, st>>>(keys, d_np, pcols_buf);
-        TSP_CUDA(cudaGetLastError());
-        pptr = pptr_buf; pcols = pcols_buf;
-    }
-    if (nseq) k_seq_tiles<<<blocks_for(nseq, T), T, 0, st>>>(nseq, pptr, seq_cls, prec, seq_tiles);
-    TSP_CUDA(cudaGetLastError());
-
-    mark("stage 4 panel lists");
     // ---- shard selection: a contiguous range of the panel sequence, balanced by tile bytes (on the device)
-    int s0 = 0, s1 = nseq, p0[3] = {0, 0, 0}, p1[3] = {totals[0], totals[1], totals[2]};
+    TspRange range_tiles("tsp convert: tiles (steps 4-7)");
+    int p0[3] = {0, 0, 0}, p1[3] = {pin->panels[0], pin->panels[1], pin->panels[2]};
+    const int nseq = p1[0] + p1[1] + p1[2];
+    int short_cls = pin->last_cls;   // class of the panel that ends at the last row of the matrix; -1: not in this shard
     h->row_begin = 0; h->row_end = rowA;
     if (shard_count > 1)
     {
-        if (nseq)
-        {
-            k_panel_costs<<<blocks_for(nseq, T), T, 0, st>>>(nseq, prec, seq_tiles, seq_cls, cost);
-            size_t bytes = cub_bytes;
-            TSP_CUDA(cub::DeviceScan::InclusiveSum(cub_tmp, bytes, cost, cost, nseq, st));
-        }
-        k_find_cuts<<<1, 32, 0, st>>>(nseq, rowA, shard_index, shard_count, cost, seq_blk, d_cuts);
-        k_shard_bounds<<<blocks_for(nseq ? nseq : 1, T) > 148 * 8 ? 148 * 8 : blocks_for(nseq ? nseq : 1, T), T, 0, st>>>(d_cuts, seq_cls, seq_idx, d_cuts);
+        double *cost;
+        int *d_cuts;
+        TSP_TRY(ws.get(&cost, nseq)); TSP_TRY(ws.get(&d_cuts, 16));
+        size_t bytes = 0;
+        TSP_CUDA(cub::DeviceScan::InclusiveSum(nullptr, bytes, cost, cost, nseq, st));
+        unsigned char *tmp;
+        TSP_TRY(ws.get(&tmp, bytes));
+        k_panel_costs<<<blocks_for(nseq, T), T, 0, st>>>(nseq, prec, seq.tiles, seq.cls, cost);
+        TSP_CUDA(cub::DeviceScan::InclusiveSum(tmp, bytes, cost, cost, nseq, st));
+        k_find_cuts<<<1, 32, 0, st>>>(nseq, rowA, shard_index, shard_count, cost, seq.blk, d_cuts);
+        k_shard_bounds<<<capped((nseq + T - 1) / T, 148 * 8), T, 0, st>>>(d_cuts, seq.cls, seq.idx, d_cuts);
         TSP_CUDA(cudaGetLastError());
-        // read-back 2 (sharded conversions only): the cuts
-        TSP_CUDA(cudaMemcpyAsync(pin, d_cuts, 10 * sizeof(int), cudaMemcpyDeviceToHost, st));
+        int *cuts = reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(pin) + sizeof(ConvStats));
+        TSP_CUDA(cudaMemcpyAsync(cuts, d_cuts, 10 * sizeof(int), cudaMemcpyDeviceToHost, st));
         TSP_CUDA(cudaStreamSynchronize(st));
-        s0 = pin[0]; s1 = pin[1];
         for (int k = 0; k < 3; k++)
         {
-            p0[k] = pin[2 + k]; p1[k] = pin[5 + k];
+            p0[k] = cuts[2 + k]; p1[k] = cuts[5 + k];
             if (p1[k] <= p0[k] || p0[k] == 0x7fffffff) { p0[k] = 0; p1[k] = 0; }
         }
-        h->row_begin = pin[8]; h->row_end = pin[9];
-        TSP_CUDA(cudaMemsetAsync(class_rows_nnz, 0, 6 * sizeof(unsigned long long), st));
-        if (s1 > s0)
+        h->row_begin = cuts[8]; h->row_end = cuts[9];
+        if (cuts[1] < nseq || cuts[0] >= cuts[1]) short_cls = -1;
+        int most = 0;
+        for (int k = 0; k < 3; k++) if (p1[k] - p0[k] > most) most = p1[k] - p0[k];
+        TSP_CUDA(cudaMemsetAsync(d_stats->max_len, 0, sizeof(ConvStats) - offsetof(ConvStats, max_len), st));
+        k_shard_stats<<<blocks_for(most, T), T, 0, st>>>(all, make_int3(p0[0], p0[1], p0[2]), make_int3(p1[0], p1[1], p1[2]), d_stats);
+        TSP_CUDA(cudaGetLastError());
+        TSP_CUDA(cudaMemcpyAsync(pin, d_stats, sizeof(ConvStats), cudaMemcpyDeviceToHost, st));
+        TSP_CUDA(cudaStreamSynchronize(st));
+    }
+    for (int k = 0; k < 3; k++)
+    {
+        TspClass &c = h->cls[k];
+        c.tilem = p1[k] - p0[k];
+        c.tilenum = pin->tiles[k];
+        c.nnz = pin->nnz[k];
+        c.rows = c.tilem * c.BM;
+        if (k == short_cls && c.tilem)   // the last panel ends with the matrix: all rows minus the other classes' full panels
         {
-            k_class_totals<<<blocks_for(s1 - s0, T) > 148 * 8 ? 148 * 8 : blocks_for(s1 - s0, T), T, 0, st>>>(s0, s1, rowA, seq_cls, seq_blk, d_rowptr,
-                                                                                                              class_rows_nnz);
-            TSP_CUDA(cudaGetLastError());
+            long long others = 0;
+            for (int q = 0; q < 3; q++) if (q != k) others += (long long)(p1[q] - p0[q]) * tsp_bm(q);
+            c.rows = (int)((long long)(h->row_end - h->row_begin) - others);
         }
-    }
-    for (int k = 0; k < 3; k++) h->cls[k].tilem = p1[k] - p0[k];
-
-    // ---- tile_ptr: tiles per panel into a workspace array per class, prefix sums; read-back 3: tiles per class
-    int *cnt[3], *prow[3], *tptr[3];
-    for (int k = 0; k < 3; k++)
-    {
-        TSP_TRY(ws.get(&cnt[k], (size_t)h->cls[k].tilem + 1)); TSP_TRY(ws.get(&prow[k], (size_t)h->cls[k].tilem + 1));
-        TSP_TRY(ws.get(&tptr[k], (size_t)h->cls[k].tilem + 1));
-        TSP_CUDA(cudaMemsetAsync(cnt[k], 0, ((size_t)h->cls[k].tilem + 1) * 4, st));
-    }
-    if (s1 > s0)
-    {
-        k_class_arrays<<<blocks_for(s1 - s0, T), T, 0, st>>>(s0, s1, seq_tiles, seq_cls, seq_idx, seq_blk, p0[0], p0[1], p0[2], cnt[0], cnt[1], cnt[2],
-                                                           prow[0], prow[1], prow[2]);
-        TSP_CUDA(cudaGetLastError());
-    }
-    for (int k = 0; k < 3; k++)
-    {
-        TspClass &c = h->cls[k];
-        size_t bytes = cub_bytes;
-        TSP_CUDA(cub::DeviceScan::ExclusiveSum(cub_tmp, bytes, cnt[k], tptr[k], c.tilem + 1, st));
-        c.h_tile_ptr.resize((size_t)c.tilem + 1);
-        c.h_panel_row.resize(c.tilem);
-        TSP_CUDA(cudaMemcpyAsync(c.h_tile_ptr.data(), tptr[k], ((size_t)c.tilem + 1) * 4, cudaMemcpyDeviceToHost, st));
-        if (c.tilem) TSP_CUDA(cudaMemcpyAsync(c.h_panel_row.data(), prow[k], (size_t)c.tilem * 4, cudaMemcpyDeviceToHost, st));
-    }
-    if (shard_count > 1) TSP_CUDA(cudaMemcpyAsync(pin + 8, class_rows_nnz, 6 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-    TSP_CUDA(cudaStreamSynchronize(st));
-    if (shard_count > 1) memcpy(tot_rows_nnz, pin + 8, sizeof(tot_rows_nnz));
-    for (int k = 0; k < 3; k++)
-    {
-        TspClass &c = h->cls[k];
-        c.tilenum = c.h_tile_ptr[c.tilem];
-        c.rows = (int)tot_rows_nnz[k * 2];
-        c.nnz = (long long)tot_rows_nnz[k * 2 + 1];
+        c.max_len = pin->max_len[k];
+        if (c.max_len < TSP_HIST_BINS - 1) c.len_hist.assign(pin->hist[k], pin->hist[k] + c.max_len + 1);
     }
 
-    mark("shards + tile_ptr + readback");
-    // ---- the tile arrays of all classes: one allocation
+    // ---- step 4: the tile arrays of all classes, one allocation
     TSP_TRY(tsp_alloc_tile_arrays(h));
-    mark("allocate + clear tile arrays");
+    mark("step 4 allocation");
+    int most = 0;
+    ClassArrays mine;
     for (int k = 0; k < 3; k++)
     {
         TspClass &c = h->cls[k];
-        TSP_CUDA(cudaMemcpyAsync(c.d_tile_ptr, tptr[k], ((size_t)c.tilem + 1) * 4, cudaMemcpyDeviceToDevice, st));
-        if (c.tilem) TSP_CUDA(cudaMemcpyAsync(c.d_panel_row, prow[k], (size_t)c.tilem * 4, cudaMemcpyDeviceToDevice, st));
+        if (c.tilem > most) most = c.tilem;
+        mine.tile_ptr[k] = c.d_tile_ptr; mine.panel_row[k] = c.d_panel_row; mine.nnz_ptr[k] = nullptr;
     }
-    if (s1 > s0)
-    {
-        const int blocks = blocks_for((long long)(s1 - s0) * 32, T) > 148 * 32 ? 148 * 32 : blocks_for((long long)(s1 - s0) * 32, T);
-        k_fill_colidx<<<blocks, T, 0, st>>>(s0, s1, prec, pptr, pcols, seq_cls, seq_idx, p0[0], p0[1], p0[2], h->cls[0].d_tile_ptr,
-                                            h->cls[1].d_tile_ptr, h->cls[2].d_tile_ptr, h->cls[0].d_tile_colidx, h->cls[1].d_tile_colidx,
-                                            h->cls[2].d_tile_colidx);
-        TSP_CUDA(cudaGetLastError());
-        // ---- stage 5
-        TSP_TRY(wait_values());
-        const int vblocks = blocks_for((long long)rowA * 32, T) > 148 * 64 ? 148 * 64 : blocks_for((long long)rowA * 32, T);
-        if (prec == 0)
-            k_place_values<__half><<<vblocks, T, 0, st>>>(rowA, 0, s0, s1, d_rowptr, d_colidx, (const __half *)d_val, blk_seq, seq_cls, seq_idx,
-                                                          seq_blk, pptr, pcols, p0[0], p0[1], p0[2], h->cls[0].d_tile_ptr, h->cls[1].d_tile_ptr,
-                                                          h->cls[2].d_tile_ptr, h->cls[0].d_tile_nnz, h->cls[1].d_tile_nnz, h->cls[2].d_tile_nnz,
-                                                          (unsigned int *)h->cls[0].d_bitmap, (__half *)h->cls[1].d_val, (__half *)h->cls[2].d_val);
-        else
-            k_place_values<float><<<vblocks, T, 0, st>>>(rowA, 1, s0, s1, d_rowptr, d_colidx, (const float *)d_val, blk_seq, seq_cls, seq_idx,
-                                                         seq_blk, pptr, pcols, p0[0], p0[1], p0[2], h->cls[0].d_tile_ptr, h->cls[1].d_tile_ptr,
-                                                         h->cls[2].d_tile_ptr, h->cls[0].d_tile_nnz, h->cls[1].d_tile_nnz, h->cls[2].d_tile_nnz,
-                                                         (unsigned int *)h->cls[0].d_bitmap, (float *)h->cls[1].d_val, (float *)h->cls[2].d_val);
-        TSP_CUDA(cudaGetLastError());
-    }
-    mark("stage 5 colidx + values");
-    for (int k = 0; k < 3; k++)  // tile_nnz: exclusive scan over tilenum+1 entries (src/csr2tile.h:786)
+    k_class_slices<<<blocks_for((long long)most + 1, T), T, 0, st>>>(all, make_int3(p0[0], p0[1], p0[2]), make_int3(p1[0], p1[1], p1[2]), mine, h->cls[0].d_tile_nnz,
+                                                                    h->cls[1].d_tile_nnz, h->cls[2].d_tile_nnz);
+    TSP_CUDA(cudaGetLastError());
+    ClassView view[3];
+    for (int k = 0; k < 3; k++)
     {
         TspClass &c = h->cls[k];
-        size_t bytes = 0;
-        TSP_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, bytes, c.d_tile_nnz, c.d_tile_nnz, c.tilenum + 1, st));
-        void *tmp = cub_tmp;
-        if (bytes > cub_bytes) { unsigned char *more; TSP_TRY(ws.get(&more, bytes)); tmp = more; }
-        TSP_CUDA(cub::DeviceScan::ExclusiveSum(tmp, bytes, c.d_tile_nnz, c.d_tile_nnz, c.tilenum + 1, st));
+        ClassView &v = view[k];
+        v.cls = k; v.tilem = c.tilem; v.tile_ptr = c.d_tile_ptr; v.panel_row = c.d_panel_row; v.nnz_ptr = all.nnz_ptr[k] + p0[k];
+        v.tile_colidx = c.d_tile_colidx; v.tile_nnz = c.d_tile_nnz;
+        // slices: at most one partly filled slice per panel that has any; 16- and 8-row panels only when they are long
+        const int per = SLICE_COLS / c.BN;
+        const long long long_panels = k == 0 ? c.tilem : c.nnz / (small_cols(prec, k) - c.BN + 1);
+        v.item_cap = (int)(c.tilenum / per + (long_panels < c.tilem ? long_panels : c.tilem));
+        v.items = nullptr;
+        if (v.item_cap > 0) TSP_TRY(ws.get(&v.items, (size_t)v.item_cap));
     }
 
-    // ---- stage 6: records of the 64-row class
+    // ---- step 5: column lists of the tall panels (the mid and big lists of step 1 are done with)
+    const int chunk_cap = (int)(h->cls[0].nnz / CHUNK_N + h->cls[0].tilem);
+    int2 *chunks = nullptr;
+    if (chunk_cap > 0) TSP_TRY(ws.get(&chunks, (size_t)chunk_cap));
+    const bool long16 = view[1].item_cap > 0;
+    if (h->cls[0].tilem > 0 || long16)
+    {
+        ClassView v16 = view[1];
+        if (!long16) v16.tilem = 0;
+        const long long keys = h->cls[0].nnz + (long16 ? h->cls[1].nnz : 0);
+        k_panel_lists<<<capped(((long long)h->cls[0].tilem + v16.tilem + 7) / 8, 148 * 32), T, 0, st>>>(nb8, rowA, prec, d_rowptr, ucols, ulen, view[0], v16, chunks, chunk_cap,
+                                                                                                       mid, big, d_stats);
+        if (keys > SMALL_N) k_panel_lists_mid<<<capped(keys / SMALL_N, 148 * 5), T, 0, st>>>(nb8, prec, bits, d_rowptr, ucols, ulen, view[0], v16, mid, d_stats);
+        if (keys > MID_N) k_panel_lists_big<<<capped(keys / MID_N, 148), 1024, words * 4, st>>>(nb8, colA, prec, words, d_rowptr, ucols, ulen, view[0], v16, big, d_stats);
+        TSP_CUDA(cudaGetLastError());
+    }
+    mark("step 5 panel lists");
+
+    // ---- step 6
+    TSP_TRY(wait_values());
+    if (prec == 0)
+    {
+        TSP_TRY((fill_class<__half, 1>(h, nb8, d_rowptr, d_colidx, (const __half *)d_val, ucols, ulen, view[1], h->cls[1].nnz, d_stats, st)));
+        TSP_TRY((fill_class<__half, 2>(h, nb8, d_rowptr, d_colidx, (const __half *)d_val, ucols, ulen, view[2], h->cls[2].nnz, d_stats, st)));
+    }
+    else
+    {
+        TSP_TRY((fill_class<float, 1>(h, nb8, d_rowptr, d_colidx, (const float *)d_val, ucols, ulen, view[1], h->cls[1].nnz, d_stats, st)));
+        TSP_TRY((fill_class<float, 2>(h, nb8, d_rowptr, d_colidx, (const float *)d_val, ucols, ulen, view[2], h->cls[2].nnz, d_stats, st)));
+    }
+    mark("step 6 16/8-row tiles");
+
+    // ---- step 7
     {
         TspClass &c = h->cls[0];
         c.d_pack = nullptr; c.pack_bytes = 0;
         if (c.tilenum > 0)
         {
             unsigned int *units, *prefix;
-            unsigned char *dense;
+            unsigned char *dense, *repeated, *tmp;
             unsigned short *row_off;
-            TSP_TRY(ws.get(&units, (size_t)c.tilenum + 1)); TSP_TRY(ws.get(&prefix, (size_t)c.tilenum + 1)); TSP_TRY(ws.get(&dense, c.tilenum));
-            TSP_TRY(ws.get(&row_off, (size_t)c.tilenum * 64));
-            TSP_CUDA(cudaMemsetAsync(units + c.tilenum, 0, 4, st));
-            const int wblocks = blocks_for((long long)c.tilenum * 32, T) > 148 * 32 ? 148 * 32 : blocks_for((long long)c.tilenum * 32, T);
-            k_rec_sizes<<<wblocks, T, 0, st>>>(c.tilenum, prec, (const unsigned int *)c.d_bitmap, units, dense, row_off);
             size_t bytes = 0;
+            TSP_TRY(ws.get(&units, (size_t)c.tilenum + 1)); TSP_TRY(ws.get(&prefix, (size_t)c.tilenum + 1)); TSP_TRY(ws.get(&dense, c.tilenum));
+            TSP_TRY(ws.get(&row_off, (size_t)c.tilenum * 64)); TSP_TRY(ws.get(&repeated, c.tilem));
             TSP_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, bytes, units, prefix, c.tilenum + 1, st));
-            void *tmp = cub_tmp;
-            if (bytes > cub_bytes) { unsigned char *more; TSP_TRY(ws.get(&more, bytes)); tmp = more; }
+            TSP_TRY(ws.get(&tmp, bytes));
+            TSP_CUDA(cudaMemsetAsync(units + c.tilenum, 0, 4, st));
+            TSP_CUDA(cudaMemsetAsync(repeated, 0, c.tilem, st));
+            const int grid = capped(view[0].item_cap, 148 * 8);
+            if (prec == 0)
+                k_masks64<0><<<grid, T, sizeof(Masks64<0>::Shared), st>>>(rowA, d_rowptr, d_colidx, view[0], (unsigned *)c.d_bitmap, units, dense, row_off, repeated, d_stats);
+            else
+                k_masks64<1><<<grid, T, sizeof(Masks64<1>::Shared), st>>>(rowA, d_rowptr, d_colidx, view[0], (unsigned *)c.d_bitmap, units, dense, row_off, repeated, d_stats);
             TSP_CUDA(cub::DeviceScan::ExclusiveSum(tmp, bytes, units, prefix, c.tilenum + 1, st));
             k_rec_finish<<<blocks_for(c.tilenum + 1, T), T, 0, st>>>(c.tilenum, prefix, dense, c.d_rec);
             TSP_CUDA(cudaGetLastError());
-            // read-back 4 (only when there are 64-row tiles): bytes of all records
+            // second read-back (only when there are 64-row tiles): bytes of all records
             TSP_CUDA(cudaMemcpyAsync(pin, prefix + c.tilenum, 4, cudaMemcpyDeviceToHost, st));
             TSP_CUDA(cudaStreamSynchronize(st));
-            const long long total_units = (unsigned int)pin[0];
+            const long long total_units = *reinterpret_cast<const unsigned int *>(pin);
             if (total_units >= 0x7fffffffLL) { tsp_set_error("convert: the 64-row tile records exceed 32 GB"); return TSP_EINVAL; }
             TSP_TRY(tsp_alloc_pack(h, total_units * 16));
-            k_init_positions<<<c.tilenum > 148 * 16 ? 148 * 16 : c.tilenum, 64, 0, st>>>(c.tilenum, prec, c.d_rec, c.d_pack);
-            const int vblocks = blocks_for((long long)rowA * 32, T) > 148 * 64 ? 148 * 64 : blocks_for((long long)rowA * 32, T);
+            k_init_positions<<<capped(c.tilenum, 148 * 16), 64, 0, st>>>(c.tilenum, prec, c.d_rec, c.d_pack);
+            const int pgrid = capped(chunk_cap, 148 * 8);
             if (prec == 0)
-                k_place_values64<__half><<<vblocks, T, 0, st>>>(rowA, 0, s0, s1, d_rowptr, d_colidx, (const __half *)d_val, blk_seq, seq_cls, seq_idx,
-                                                                seq_blk, pptr, pcols, p0[0], c.d_tile_ptr, (const unsigned int *)c.d_bitmap, row_off,
-                                                                c.d_rec, (__half *)c.d_pack);
+                k_place_values64<__half><<<pgrid, T, 0, st>>>(rowA, d_rowptr, d_colidx, (const __half *)d_val, view[0], chunks, chunk_cap, (const unsigned *)c.d_bitmap,
+                                                              row_off, c.d_rec, repeated, (__half *)c.d_pack, d_stats);
             else
-                k_place_values64<float><<<vblocks, T, 0, st>>>(rowA, 1, s0, s1, d_rowptr, d_colidx, (const float *)d_val, blk_seq, seq_cls, seq_idx,
-                                                               seq_blk, pptr, pcols, p0[0], c.d_tile_ptr, (const unsigned int *)c.d_bitmap, row_off,
-                                                               c.d_rec, (float *)c.d_pack);
+                k_place_values64<float><<<pgrid, T, 0, st>>>(rowA, d_rowptr, d_colidx, (const float *)d_val, view[0], chunks, chunk_cap, (const unsigned *)c.d_bitmap,
+                                                             row_off, c.d_rec, repeated, (float *)c.d_pack, d_stats);
             TSP_CUDA(cudaGetLastError());
         }
     }
     TSP_CUDA(cudaStreamSynchronize(st));
-    mark("stage 6 records");
+    mark("step 7 64-row records");
     // a large workspace (hundreds of millions of entries) is given back; a small one stays for the next conversion
     size_t held = 0;
     for (auto &ch : h->ws_chunks) held += ch.second;

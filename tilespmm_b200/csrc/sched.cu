@@ -56,13 +56,75 @@ __global__ void k_task_fill(int tilem, const int *__restrict__ tile_ptr, const i
     split_row[atomicAdd(split_count, 1)] = row;
 }
 
-// sort key of a task: longer tasks get smaller keys
-__global__ void k_task_keys(int ntasks, const int *__restrict__ task_start, unsigned int *__restrict__ keys, int *__restrict__ ids)
+// One class in one CTA, for at most SCHED_PANELS panels and SCHED_TASKS tasks: task counts, their prefix sum, the tasks,
+// and (pack != nullptr) the same tasks longest first.  Small matrices pay for launches, not for work: this is one launch
+// where the general path below takes seven.
+constexpr int SCHED_T = 512, SCHED_PANELS = 2048, SCHED_TASKS = 2048;
+__global__ void __launch_bounds__(SCHED_T) k_schedule_small(int tilem, const int *__restrict__ tile_ptr, const int *__restrict__ panel_row, int TH, int sorted,
+                                                         unsigned int *__restrict__ task_row, int *__restrict__ task_start, int *__restrict__ split_row, uint4 *__restrict__ pack)
+{
+    using Scan = cub::BlockScan<int, SCHED_T>;
+    using Sort = cub::BlockRadixSort<unsigned, SCHED_T, SCHED_TASKS / SCHED_T>;
+    __shared__ union { Scan::TempStorage scan; Sort::TempStorage sort; } temp;
+    __shared__ int starts[SCHED_TASKS + 1], s_split;
+    __shared__ unsigned rows[SCHED_TASKS];
+    const int tid = threadIdx.x;
+    constexpr int PER = SCHED_PANELS / SCHED_T;
+    int t0[PER], len[PER], parts[PER], mine = 0, ntasks;
+    if (tid == 0) s_split = 0;
+#pragma unroll
+    for (int i = 0; i < PER; i++)
+    {
+        const int p = tid * PER + i;
+        t0[i] = p < tilem ? tile_ptr[p] : 0;
+        len[i] = p < tilem ? tile_ptr[p + 1] - t0[i] : 0;
+        parts[i] = p < tilem ? (len[i] <= TH ? 1 : (len[i] + TH - 1) / TH) : 0;   // src/csr2tile.h:392-396
+        mine += parts[i];
+    }
+    int b;
+    Scan(temp.scan).ExclusiveSum(mine, b, ntasks);
+#pragma unroll
+    for (int i = 0; i < PER; i++)
+    {
+        const int p = tid * PER + i;
+        if (p >= tilem) break;
+        const int row = panel_row[p];
+        const int each = (len[i] + parts[i] - 1) / parts[i];   // src/csr2tile.h:421-422
+        if (parts[i] > 1) split_row[atomicAdd(&s_split, 1)] = row;
+        for (int s = 0; s < parts[i]; s++, b++)
+        {
+            rows[b] = (unsigned)row | (parts[i] > 1 ? 0x80000000u : 0u);
+            starts[b] = t0[i] + s * each;
+        }
+        if (p == tilem - 1) starts[b] = t0[i] + len[i];
+    }
+    __syncthreads();
+    for (int t = tid; t < ntasks; t += SCHED_T) task_row[t] = rows[t];
+    for (int t = tid; t <= ntasks; t += SCHED_T) task_start[t] = starts[t];
+    if (!pack) return;
+    unsigned key[SCHED_TASKS / SCHED_T];
+#pragma unroll
+    for (int i = 0; i < SCHED_TASKS / SCHED_T; i++)
+    {
+        const int t = tid * (SCHED_TASKS / SCHED_T) + i;
+        key[i] = t < ntasks ? (0xffffu - (unsigned)min(starts[t + 1] - starts[t], 0xffff)) << 16 | (unsigned)t : 0xffffffffu;
+    }
+    if (sorted) Sort(temp.sort).Sort(key, 16, 32);
+#pragma unroll
+    for (int i = 0; i < SCHED_TASKS / SCHED_T; i++)
+    {
+        const int at = tid * (SCHED_TASKS / SCHED_T) + i, t = (int)(key[i] & 0xffffu);
+        if (at < ntasks) pack[at] = make_uint4(rows[t], (unsigned)starts[t], (unsigned)starts[t + 1], 0u);
+    }
+}
+
+// sort key of a task: longer tasks get smaller keys (`top` bounds the lengths; the keys need bits_of(top) bits)
+__global__ void k_task_keys(int ntasks, unsigned top, const int *__restrict__ task_start, unsigned int *__restrict__ keys, int *__restrict__ ids)
 {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= ntasks) return;
-    const int len = task_start[t + 1] - task_start[t];
-    keys[t] = 0xffffu - (unsigned int)(len > 0xffff ? 0xffff : len);
+    const unsigned len = (unsigned)(task_start[t + 1] - task_start[t]);
+    keys[t] = top - (len > top ? top : len);
     ids[t] = t;
 }
 
@@ -79,51 +141,60 @@ __global__ void k_task_pack(int ntasks, const int *__restrict__ order, const uns
 // task is done.  Walking the tasks longest first (stable, so equal tasks keep their panel order and with it the
 // locality of their B rows in L2) puts tasks of similar length into one CTA and the long ones at the front of the
 // launch.  TSP_TASK_ORDER=0 in the environment keeps panel order.
-int build_task_pack(TspClass &c)
+bool tasks_sorted()
 {
-    if (c.ntasks == 0) return TSP_OK;
-    static int sorted = -1;
-    if (sorted < 0) { const char *e = getenv("TSP_TASK_ORDER"); sorted = (e && e[0] == '0') ? 0 : 1; }
-    const int T = 256, n = c.ntasks;
-    unsigned int *keys = nullptr, *keys_out = nullptr;
-    int *ids = nullptr, *ids_out = nullptr;
-    void *scratch = nullptr;
-    cudaError_t e = cudaSuccess;
-    if (sorted)
+    static const bool sorted = [] { const char *e = getenv("TSP_TASK_ORDER"); return !(e && e[0] == '0'); }();
+    return sorted;
+}
+
+// device scratch of the schedule, kept in the handle and grown on demand
+int sched_scratch(tsp_handle *h, size_t bytes, unsigned char **p)
+{
+    if (bytes > h->sched_scratch_bytes)
     {
-        size_t bytes = 0;
-        e = cudaMalloc((void **)&keys, (size_t)n * 16);   // keys, sorted keys, ids, sorted ids
-        if (e == cudaSuccess)
-        {
-            keys_out = keys + n; ids = (int *)(keys + 2 * (size_t)n); ids_out = ids + n;
-            k_task_keys<<<(n + T - 1) / T, T>>>(n, c.d_task_start, keys, ids);
-            e = cub::DeviceRadixSort::SortPairs(nullptr, bytes, keys, keys_out, ids, ids_out, n, 0, 16);
-        }
-        if (e == cudaSuccess) e = cudaMalloc(&scratch, bytes ? bytes : 1);
-        if (e == cudaSuccess) e = cub::DeviceRadixSort::SortPairs(scratch, bytes, keys, keys_out, ids, ids_out, n, 0, 16);
+        cudaFree(h->sched_scratch);   // waits for whatever still uses it
+        h->sched_scratch = nullptr; h->sched_scratch_bytes = 0;
+        TSP_CUDA(cudaMalloc(&h->sched_scratch, bytes + bytes / 4));
+        h->sched_scratch_bytes = bytes + bytes / 4;
     }
-    if (e == cudaSuccess)
-    {
-        k_task_pack<<<(n + T - 1) / T, T>>>(n, sorted ? ids_out : nullptr, c.d_task_row, c.d_task_start, c.d_task_pack);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cudaDeviceSynchronize();   // the scratch goes away below
-    cudaFree(scratch); cudaFree(keys);
-    TSP_CUDA(e);
+    *p = static_cast<unsigned char *>(h->sched_scratch);
+    return TSP_OK;
+}
+
+// panels by number of tiles, from the conversion's histogram or from tile_ptr
+int length_histogram(const tsp_handle *h, int cls, std::vector<int> &hist)
+{
+    const TspClass &c = h->cls[cls];
+    if (!c.len_hist.empty()) { hist = c.len_hist; return TSP_OK; }
+    TSP_TRY(tsp_fetch_panels(h, cls));
+    const std::vector<int> &tp = c.h_tile_ptr;
+    int max_len = 0;
+    for (int p = 0; p < c.tilem; p++) max_len = tp[p + 1] - tp[p] > max_len ? tp[p + 1] - tp[p] : max_len;
+    hist.assign((size_t)max_len + 1, 0);
+    for (int p = 0; p < c.tilem; p++) hist[tp[p + 1] - tp[p]]++;
     return TSP_OK;
 }
 
 }  // namespace
 
-int tsp_schedule(tsp_handle *h, int cls, int TH)
+// Enqueues the task arrays of class cls for threshold TH on `s`.  How many tasks and split panels there will be follows
+// from the histogram of panel lengths, so nothing is read back and the host does not wait.
+int tsp_schedule_on(tsp_handle *h, int cls, int TH, cudaStream_t s)
 {
-    if (!h || cls < 0 || cls > 2 || TH <= 0) { tsp_set_error("schedule: bad argument"); return TSP_EINVAL; }
-    if (!h->converted) { tsp_set_error("schedule: convert first"); return TSP_ESTATE; }
-    TSP_CUDA(cudaSetDevice(h->device));
     TspRange range("tsp schedule");
     TspClass &c = h->cls[cls];
     c.TH = TH; c.ntasks = 0; c.nsplit = 0;
     if (c.tilem == 0) return TSP_OK;
+    std::vector<int> hist;
+    TSP_TRY(length_histogram(h, cls, hist));
+    long long ntasks = 0, nsplit = 0;
+    for (size_t len = 0; len < hist.size(); len++)
+    {
+        const long long parts = (long long)len <= TH ? 1 : ((long long)len + TH - 1) / TH;
+        ntasks += parts * hist[len];
+        if (parts > 1) nsplit += hist[len];
+    }
+    if (ntasks > 0x7fffffffLL) { tsp_set_error("schedule: %lld tasks", ntasks); return TSP_EINVAL; }
     if (!c.d_task_count || c.tilem > c.cap_panels)
     {
         cudaFree(c.d_task_count); cudaFree(c.d_split_row);
@@ -132,35 +203,67 @@ int tsp_schedule(tsp_handle *h, int cls, int TH)
         TSP_CUDA(cudaMalloc((void **)&c.d_split_row, ((size_t)c.tilem + 1) * 4));
         c.cap_panels = c.tilem;
     }
-    const int T = 256;
-    k_task_counts<<<(c.tilem + 1 + T - 1) / T, T>>>(c.tilem, c.d_tile_ptr, TH, c.d_task_count);
-    TSP_CUDA(cudaGetLastError());
-    size_t bytes = 0;
-    TSP_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, bytes, c.d_task_count, c.d_task_count, c.tilem + 1));
-    void *scratch = nullptr;
-    TSP_CUDA(cudaMalloc(&scratch, bytes ? bytes : 1));
-    cudaError_t e = cub::DeviceScan::ExclusiveSum(scratch, bytes, c.d_task_count, c.d_task_count, c.tilem + 1);
-    int ntasks = 0;
-    if (e == cudaSuccess) e = cudaMemcpy(&ntasks, c.d_task_count + c.tilem, 4, cudaMemcpyDeviceToHost);
-    cudaFree(scratch);
-    TSP_CUDA(e);
-    if ((long long)ntasks > c.cap_tasks)
+    if (ntasks > c.cap_tasks)
     {
         cudaFree(c.d_task_row); cudaFree(c.d_task_start); cudaFree(c.d_task_pack);
         c.d_task_row = nullptr; c.d_task_start = nullptr; c.d_task_pack = nullptr;
-        c.cap_tasks = (long long)ntasks + ntasks / 4 + 16;
-        TSP_CUDA(cudaMalloc((void **)&c.d_task_row, (size_t)c.cap_tasks * 4));
-        TSP_CUDA(cudaMalloc((void **)&c.d_task_start, ((size_t)c.cap_tasks + 1) * 4));
-        if (cls != 0) TSP_CUDA(cudaMalloc((void **)&c.d_task_pack, (size_t)c.cap_tasks * sizeof(uint4)));
+        c.cap_tasks = 0;
+        const long long cap = ntasks + ntasks / 4 + 16;
+        TSP_CUDA(cudaMalloc((void **)&c.d_task_row, (size_t)cap * 4));
+        TSP_CUDA(cudaMalloc((void **)&c.d_task_start, ((size_t)cap + 1) * 4));
+        if (cls != 0) TSP_CUDA(cudaMalloc((void **)&c.d_task_pack, (size_t)cap * sizeof(uint4)));
+        c.cap_tasks = cap;
     }
+    const int T = 256, n = (int)ntasks;
+    const bool sorted = tasks_sorted();
+    if (c.tilem <= SCHED_PANELS && n <= SCHED_TASKS)
+    {
+        k_schedule_small<<<1, SCHED_T, 0, s>>>(c.tilem, c.d_tile_ptr, c.d_panel_row, TH, sorted ? 1 : 0, c.d_task_row, c.d_task_start, c.d_split_row,
+                                           cls != 0 ? c.d_task_pack : nullptr);
+        TSP_CUDA(cudaGetLastError());
+        c.ntasks = n; c.nsplit = (int)nsplit;
+        return TSP_OK;
+    }
+    // task lengths are at most TH and at most the longest panel: one pass of the sort for lengths below 256
+    unsigned top = (unsigned)(hist.size() - 1 < (size_t)TH ? hist.size() - 1 : (size_t)TH);
+    if (top > 0xffffu) top = 0xffffu;
+    int key_bits = 1;
+    while (key_bits < 16 && (top >> key_bits)) key_bits++;
+    size_t scan_bytes = 0, sort_bytes = 0;
+    unsigned *keys = nullptr, *keys_out = nullptr;
+    int *ids = nullptr, *ids_out = nullptr;
+    TSP_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, c.d_task_count, c.d_task_count, c.tilem + 1, s));
+    const bool sorting = cls != 0 && sorted;
+    if (sorting) TSP_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, keys, keys_out, ids, ids_out, n, 0, key_bits, s));
+    size_t cub_bytes = (scan_bytes > sort_bytes ? scan_bytes : sort_bytes) + 256;
+    cub_bytes = (cub_bytes + 255) & ~(size_t)255;
+    unsigned char *scratch;
+    TSP_TRY(sched_scratch(h, cub_bytes + (sorting ? (size_t)n * 16 : 0), &scratch));
+    k_task_counts<<<(c.tilem + 1 + T - 1) / T, T, 0, s>>>(c.tilem, c.d_tile_ptr, TH, c.d_task_count);
+    TSP_CUDA(cub::DeviceScan::ExclusiveSum(scratch, scan_bytes, c.d_task_count, c.d_task_count, c.tilem + 1, s));
     int *d_split_count = c.d_task_count + c.tilem + 1;
-    TSP_CUDA(cudaMemset(d_split_count, 0, 4));
-    k_task_fill<<<(c.tilem + T - 1) / T, T>>>(c.tilem, c.d_tile_ptr, c.d_panel_row, TH, c.d_task_count, c.d_task_row, c.d_task_start,
-                                             c.d_split_row, d_split_count);
+    TSP_CUDA(cudaMemsetAsync(d_split_count, 0, 4, s));
+    k_task_fill<<<(c.tilem + T - 1) / T, T, 0, s>>>(c.tilem, c.d_tile_ptr, c.d_panel_row, TH, c.d_task_count, c.d_task_row, c.d_task_start,
+                                                   c.d_split_row, d_split_count);
+    if (sorting)
+    {
+        keys = (unsigned *)(scratch + cub_bytes); keys_out = keys + n; ids = (int *)(keys + 2 * (size_t)n); ids_out = ids + n;
+        k_task_keys<<<(n + T - 1) / T, T, 0, s>>>(n, top, c.d_task_start, keys, ids);
+        TSP_CUDA(cub::DeviceRadixSort::SortPairs(scratch, sort_bytes, keys, keys_out, ids, ids_out, n, 0, key_bits, s));
+    }
+    if (cls != 0) k_task_pack<<<(n + T - 1) / T, T, 0, s>>>(n, sorting ? ids_out : nullptr, c.d_task_row, c.d_task_start, c.d_task_pack);
     TSP_CUDA(cudaGetLastError());
-    TSP_CUDA(cudaMemcpy(&c.nsplit, d_split_count, 4, cudaMemcpyDeviceToHost));
-    c.ntasks = ntasks;
-    if (cls != 0) TSP_TRY(build_task_pack(c));
+    c.ntasks = n; c.nsplit = (int)nsplit;
+    return TSP_OK;
+}
+
+int tsp_schedule(tsp_handle *h, int cls, int TH)
+{
+    if (!h || cls < 0 || cls > 2 || TH <= 0) { tsp_set_error("schedule: bad argument"); return TSP_EINVAL; }
+    if (!h->converted) { tsp_set_error("schedule: convert first"); return TSP_ESTATE; }
+    TSP_CUDA(cudaSetDevice(h->device));
+    TSP_TRY(tsp_schedule_on(h, cls, TH, 0));
+    TSP_CUDA(cudaStreamSynchronize(0));
     return TSP_OK;
 }
 
@@ -210,18 +313,11 @@ int tsp_top4(const tsp_handle *h, int cls, int colB, int *top4)
     const float lambda_atom = tsp_atom_weight(is_tf32, cls, colB);
     const float atom_per_col = lambda_atom * (1.0f / 32.0f);
 
-    const std::vector<int> &tp = c.h_tile_ptr;
-    int max_len = 0;
-    long long total_len = 0;
-    for (int p = 0; p < c.tilem; p++)
-    {
-        const int len = tp[p + 1] - tp[p];
-        if (len > max_len) max_len = len;
-        total_len += len;
-    }
-    if (max_len == 0) return TSP_OK;
-    std::vector<int> hist((size_t)max_len + 1, 0);
-    for (int p = 0; p < c.tilem; p++) hist[tp[p + 1] - tp[p]]++;
+    std::vector<int> hist;
+    TSP_TRY(length_histogram(h, cls, hist));
+    const int max_len = (int)hist.size() - 1;
+    const long long total_len = c.tilenum;
+    if (max_len <= 0) return TSP_OK;
     hist[0] = 0;
     std::vector<int> lens;
     for (int len = 1; len <= max_len; len++) if (hist[len]) lens.push_back(len);

@@ -68,6 +68,7 @@ extern "C" int tsp_save(const tsp_handle *h, const char *path)
     for (int k = 0; k < 3 && rc == TSP_OK; k++)
     {
         const TspClass &c = h->cls[k];
+        if ((rc = tsp_fetch_panels(h, k)) != TSP_OK) break;
         if (fwrite(c.h_tile_ptr.data(), 4, (size_t)c.tilem + 1, f) != (size_t)c.tilem + 1) rc = TSP_EINVAL;
         if (rc == TSP_OK && c.tilem && fwrite(c.h_panel_row.data(), 4, (size_t)c.tilem, f) != (size_t)c.tilem) rc = TSP_EINVAL;
         if (rc == TSP_OK) rc = write_dev(f, c.d_tile_nnz, ((size_t)c.tilenum + 1) * 4, tmp);

@@ -128,6 +128,8 @@ struct TspKernelResources  // what the platform probe records per (class, width)
     long long shared_bytes;
 };
 
+#define TSP_HIST_BINS 1024
+
 struct TspClass
 {
     int BM = 0, BN = 0;
@@ -143,7 +145,11 @@ struct TspClass
     unsigned int *d_rec = nullptr;
     unsigned char *d_pack = nullptr;
     long long pack_bytes = 0;
-    std::vector<int> h_tile_ptr, h_panel_row;
+    mutable std::vector<int> h_tile_ptr, h_panel_row;   // host copies, fetched on first use (tsp_fetch_panels)
+    // panels by number of tiles (index = tiles), what the threshold model and the schedule sizes are computed from; empty
+    // when a panel is too long for it (max_len >= TSP_HIST_BINS - 1) or after tsp_load: then h_tile_ptr serves
+    std::vector<int> len_hist;
+    int max_len = 0;
     // schedule for the current threshold
     int TH = 0, ntasks = 0, nsplit = 0;
     long long cap_tasks = 0, cap_panels = 0;   // capacities of the task arrays / the per-panel arrays (kept across conversions)
@@ -174,6 +180,13 @@ struct tsp_handle
     // host buffer for the few scalars a conversion reads back
     std::vector<std::pair<void *, size_t>> ws_chunks;
     void *h_pin = nullptr;
+    void *sched_scratch = nullptr;    // device scratch of tsp_schedule_on, grown on demand
+    size_t sched_scratch_bytes = 0;
+    // A schedule that tsp_spmm builds by itself is enqueued on the caller's stream; until it is known to be complete, calls
+    // on other streams wait for this event.
+    cudaEvent_t sched_ready = nullptr;
+    cudaStream_t sched_stream = nullptr;
+    bool sched_pending = false;
     // device staging of the host-buffer entry points: two slots, so that the upload of one call overlaps the
     // download of the previous one (PCIe is full duplex); one stream per direction plus a compute stream
     void *stage_b[2] = {nullptr, nullptr};
@@ -200,9 +213,11 @@ int tsp_export_values_upstream(const tsp_handle *h, int cls, void *h_dst);
 int tsp_alloc_tile_arrays(tsp_handle *h);
 int tsp_alloc_pack(tsp_handle *h, long long bytes);
 void tsp_free_workspace(tsp_handle *h);
+int tsp_fetch_panels(const tsp_handle *h, int cls);   // fills h_tile_ptr and h_panel_row of one class
 
-// class kernels; C is addressed relative to row_begin.  count_only != 0 skips the launch and only reports
-// how many launches the call would make.
+int tsp_schedule_on(tsp_handle *h, int cls, int TH, cudaStream_t s);   // enqueues only
+
+// class kernels; C is addressed relative to row_begin
 int tsp_launch_class64(tsp_handle *h, const void *d_b, float *d_c, int colB, cudaStream_t s);
 int tsp_launch_class64_tma(tsp_handle *h, const void *d_b, float *d_c, int colB, cudaStream_t s);
 int tsp_launch_small(tsp_handle *h, int cls, const void *d_b, float *d_c, int colB, cudaStream_t s);
