@@ -52,6 +52,33 @@ def test_conversion_at_the_edges_of_its_methods(prec, cols, repeats):
     m.close()
 
 
+@pytest.mark.parametrize("blocks", [1, 7, 63, 64, 65, 511, 512, 513, 1100])
+def test_panel_chain_at_the_edges_of_its_chunks(blocks):
+    """The chain of panels is resolved in chunks of 64 8-row blocks, eight chunks per CTA: panels of all heights across both
+    edges, a last chunk shorter than a tall panel, a last block of three rows."""
+    from tilespmm_b200 import api
+    rng = np.random.default_rng(blocks)
+    rows, cols = 8 * blocks - 5, 900
+    lens, ci, style, pool = [], [], 0, None
+    for r in range(rows):
+        if r % 8 == 0 and (r == 0 or rng.random() < 0.3):
+            style, pool = rng.integers(0, 4), rng.choice(cols, size=24, replace=False)
+        c = rng.permutation(pool)[:12] if style < 2 else rng.choice(cols, size=(0 if style == 2 and rng.random() < 0.2 else 6), replace=False)
+        lens.append(c.size)
+        ci.append(c.astype(np.int32))
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    ci = np.concatenate(ci).astype(np.int32)
+    v, m = api.to_values(rng.uniform(-1.0, 1.0, size=ci.size).astype(np.float32), 1), api.TileMatrix(1)
+    for g, d in ((2.0, 1.2), (3.0, 1.5), (4.0, 1.4), (0.0, 1.5), (5.0, 0.0), (5.0, 3.0)):
+        m.convert_host((rows, cols), rp, ci, v, g, d)
+        o = _orc.Orc(1, (rows, cols), rp, ci, v, g, d)
+        assert m.info().tolist() == o.info().tolist(), (g, d)
+        for cls in range(3):
+            for w in _orc.ARRAYS:
+                np.testing.assert_array_equal(m.array(cls, w), o.array(cls, w), err_msg=f"{g},{d} class {cls} {w}")
+    m.close()
+
+
 @pytest.mark.parametrize("tasks", [2047, 2048, 2049, 70000])
 def test_schedule_at_the_edge_of_the_one_block_builder(tasks):
     """Up to 2048 panels and tasks one CTA builds the schedule; the task list and the walked copy must cover the same tiles."""

@@ -453,42 +453,93 @@ __global__ void __launch_bounds__(256) k_fresh_columns(int nb8, int rowA, int nn
 
 __device__ __forceinline__ int step_of(int cls) { return cls == 0 ? 8 : (cls == 1 ? 2 : 1); }
 
-constexpr int LOCAL_CHUNKS = 8;     // chunks per CTA of k_chain_local
-constexpr int EMIT_CHUNKS = 32;     // chunks per CTA of k_chain_emit
+constexpr int CHAIN_CHUNKS = 8;     // chunks per CTA of the chain kernels
+constexpr int CHAIN_NB = CHAIN_CHUNKS * CHAIN_L;   // a thread per block
 constexpr int CHAIN_N = 9;          // panels, tiles and entries of the three classes
 
-// The chain i <- i + step(i) is resolved chunk-wise.  Chunks are short (CHAIN_L blocks) and staged in shared memory, so
-// that a walk costs shared-memory latency per step; the chunks are then linked by a parallel scan over "entry offset ->
+// For every block of a chunk: where the chain that passes it leaves the chunk and what it passes from there on (the
+// block's own panel included), by doubling: six rounds in which a thread appends its successor's stretch to its own.  A
+// thread that walked the 64 blocks one after the other took 15 - 35 us for the two chain kernels, whatever the size of the
+// matrix (4096 rows: 15 + 13 us, 262144 rows: 17 + 34 us); this takes 6 + 8 us
+// and 6 + 10 us.
+struct ChainTails
+{
+    int panels[CHAIN_NB];           // panels of the three classes, 8 bits each (a chunk has 64 blocks)
+    int tiles[3][CHAIN_NB], nnz[3][CHAIN_NB];
+    unsigned char next[CHAIN_NB];
+
+    __device__ __forceinline__ void store(const int (&v)[7], int nx)
+    {
+        const int i = threadIdx.x;
+        panels[i] = v[0];
+#pragma unroll
+        for (int q = 0; q < 3; q++) { tiles[q][i] = v[1 + q]; nnz[q][i] = v[4 + q]; }
+        next[i] = (unsigned char)nx;
+    }
+    // counts of the tail that starts at block i of this CTA
+    __device__ __forceinline__ void counts(int i, int (&c)[CHAIN_N]) const
+    {
+#pragma unroll
+        for (int q = 0; q < 3; q++) { c[q] = panels[i] >> (8 * q) & 0xff; c[3 + q] = tiles[q][i]; c[6 + q] = nnz[q][i]; }
+    }
+    // called by all CHAIN_NB threads: block `pos` of a chunk of `len` blocks starts a panel of class k with tl tiles and en entries
+    __device__ __forceinline__ void build(int pos, int len, int k, int tl, int en)
+    {
+        const bool on = pos < len;
+        int v[7], nx = on ? pos + step_of(k) : CHAIN_L + 8;
+        v[0] = on ? 1 << (8 * k) : 0;
+#pragma unroll
+        for (int q = 0; q < 3; q++) { v[1 + q] = on && q == k ? tl : 0; v[4 + q] = on && q == k ? en : 0; }
+        const int chunk0 = (int)threadIdx.x & ~(CHAIN_L - 1);
+        for (int round = 0; round < 6; round++)   // after round r a stretch has up to 2^(r+1) panels; 64 end every chunk
+        {
+            store(v, nx);
+            __syncthreads();
+            if (nx < len)
+            {
+                const int i = chunk0 + nx;
+                v[0] += panels[i];
+#pragma unroll
+                for (int q = 0; q < 3; q++) { v[1 + q] += tiles[q][i]; v[4 + q] += nnz[q][i]; }
+                nx = next[i];
+            }
+            __syncthreads();
+        }
+        store(v, nx);
+        __syncthreads();
+    }
+};
+static_assert(CHAIN_L == 64, "six rounds, 8-bit panel counts, two warps per chunk");
+
+// The chain i <- i + step(i) is resolved chunk-wise; the chunks are then linked by a parallel scan over "entry offset ->
 // exit offset" tables (8 states), not by a serial pass.
 //
 // This kernel: the class every start would take and the tiles its panel would have; then, for every chunk and every entry
 // offset 0..7, where the chain leaves the chunk and how many panels, tiles and entries of each class it passes.
-__global__ void __launch_bounds__(LOCAL_CHUNKS * 8)
+__global__ void __launch_bounds__(CHAIN_NB)
 k_chain_local(int nb8, int nchunk, int rowA, int nnz, int precision, float gamma, float delta, int fixed, int reach, const int *__restrict__ rowptr,
               const int *__restrict__ ulen, const int *__restrict__ fresh, unsigned char *__restrict__ cls_of, int *__restrict__ tiles_of,
               unsigned char *__restrict__ exit_off, int *__restrict__ counts /* [nchunk*8][CHAIN_N] */)
 {
-    constexpr int NB = LOCAL_CHUNKS * CHAIN_L;
-    __shared__ int n16_s[NB + 8], rp_s[NB + 9], tiles_s[NB];
-    __shared__ unsigned char cls_s[NB];
-    const int first = blockIdx.x * NB, tid = threadIdx.x;
-    for (int i = tid; i < NB + 9; i += LOCAL_CHUNKS * 8)
+    __shared__ int n16_s[CHAIN_NB + 8], rp_s[CHAIN_NB + 9];
+    __shared__ ChainTails tails;
+    const int first = blockIdx.x * CHAIN_NB, tid = threadIdx.x;
+    for (int i = tid; i < CHAIN_NB + 9; i += CHAIN_NB)
     {
         const int b = first + i;
         rp_s[i] = min(max(rowptr[b < nb8 ? b * 8 : rowA], 0), nnz);
-        if (i < NB + 8 && reach > 0) n16_s[i] = b < nb8 ? fresh[b * 8] + fresh[b * 8 + 9] : 0;
+        if (i < CHAIN_NB + 8 && reach > 0) n16_s[i] = b < nb8 ? fresh[b * 8] + fresh[b * 8 + 9] : 0;
     }
     __syncthreads();
-    for (int i = tid; i < NB; i += LOCAL_CHUNKS * 8)
+    const int b = first + tid;
+    int k = 2, tl = 0;
+    if (b < nb8)
     {
-        const int b = first + i;
-        if (b >= nb8) break;
         const long long row = (long long)b * 8;
         int N64 = 0;
         if (reach == 7)
 #pragma unroll
             for (int q = 0; q < 8; q++) N64 += b + q < nb8 ? fresh[(b + q) * 8 + q] : 0;
-        int k = 2;
         if (fixed >= 0) k = fixed;   // src/hetero_split.h:152-169
         else
         {
@@ -499,42 +550,34 @@ k_chain_local(int nb8, int nchunk, int rowA, int nnz, int precision, float gamma
                 int s16 = 0;
                 for (int q = 0; q < 4 && !is64; q++)
                 {
-                    s16 += n16_s[i + 2 * q];
+                    s16 += n16_s[tid + 2 * q];
                     if ((float)s16 > thr) is64 = true;
                 }
             }
             if (is64) k = 0;
             else if (delta <= 0.0f) k = 1;
-            else if (!(delta > 2.0f) && row + 16 <= rowA && n16_s[i] > 0)
+            else if (!(delta > 2.0f) && row + 16 <= rowA && n16_s[tid] > 0)
             {
-                const float thr = delta * n16_s[i];
+                const float thr = delta * n16_s[tid];
                 int s8 = ulen[b];
                 bool is16 = (float)s8 >= thr;
                 if (!is16) { s8 += ulen[b + 1]; is16 = (float)s8 >= thr; }
                 if (is16) k = 1;
             }
         }
-        const int d = k == 0 ? N64 : (k == 1 ? n16_s[i] : ulen[b]), bn = tsp_bn(precision, k);
-        cls_s[i] = (unsigned char)k; tiles_s[i] = (d + bn - 1) / bn;   // src/csr2tile.h:45-46
-        cls_of[b] = (unsigned char)k; tiles_of[b] = tiles_s[i];
+        const int d = k == 0 ? N64 : (k == 1 ? n16_s[tid] : ulen[b]), bn = tsp_bn(precision, k);
+        tl = (d + bn - 1) / bn;   // src/csr2tile.h:45-46
+        cls_of[b] = (unsigned char)k; tiles_of[b] = tl;
     }
-    __syncthreads();
-    const int t = blockIdx.x * LOCAL_CHUNKS * 8 + tid;
-    if (t >= nchunk * 8) return;
-    const int c = t >> 3, o = t & 7, base = (tid >> 3) * CHAIN_L;
-    const int len = min(CHAIN_L, nb8 - c * CHAIN_L);
-    int pos = o, cnt[CHAIN_N] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    while (pos < len)
-    {
-        const int k = cls_s[base + pos], st = step_of(k), tl = tiles_s[base + pos], en = rp_s[base + pos + st] - rp_s[base + pos];
+    const int c = b / CHAIN_L, pos = b % CHAIN_L, len = min(CHAIN_L, nb8 - c * CHAIN_L);
+    tails.build(pos, len, k, tl, rp_s[tid + step_of(k)] - rp_s[tid]);
+    if (c >= nchunk || pos >= 8) return;
+    const int off = pos < len ? (int)tails.next[tid] - CHAIN_L : 0;
+    exit_off[c * 8 + pos] = (unsigned char)(off < 0 ? 0 : (off > 7 ? 7 : off));
+    int cnt[CHAIN_N];
+    tails.counts(tid, cnt);   // zero behind the last block
 #pragma unroll
-        for (int q = 0; q < 3; q++) if (q == k) { cnt[q]++; cnt[3 + q] += tl; cnt[6 + q] += en; }
-        pos += st;
-    }
-    const int off = pos - CHAIN_L;
-    exit_off[t] = (unsigned char)(off < 0 ? 0 : (off > 7 ? 7 : off));
-#pragma unroll
-    for (int q = 0; q < CHAIN_N; q++) counts[t * CHAIN_N + q] = cnt[q];
+    for (int q = 0; q < CHAIN_N; q++) counts[(c * 8 + pos) * CHAIN_N + q] = cnt[q];
 }
 
 // Links the chunks: the entry offset of every chunk (composition of the chunks' transition tables, 8 states of 3 bits
@@ -640,57 +683,70 @@ struct SeqArrays
     unsigned char *cls;
 };
 
-// Walks every chunk from its true entry and writes its panels.  One thread per chunk, 32 chunks per CTA.
-__global__ void __launch_bounds__(128)
+// Writes the panels of every chunk.  One thread per chunk follows the chain from its true entry and marks the blocks that
+// start panels; then every block knows from the tails what lies between the entry and itself.
+__global__ void __launch_bounds__(CHAIN_NB)
 k_chain_emit(int nb8, int nchunk, int rowA, int nnz, const unsigned char *__restrict__ cls_of, const int *__restrict__ tiles_of,
              const int *__restrict__ entry, const int *__restrict__ base, const int *__restrict__ rowptr, ClassArrays out, SeqArrays seq, ConvStats *st)
 {
-    constexpr int NB = EMIT_CHUNKS * CHAIN_L;
-    __shared__ unsigned char cls_s[NB];
-    __shared__ int tiles_s[NB], rp_s[NB + 8];
+    __shared__ unsigned char cls_s[CHAIN_NB];
+    __shared__ ChainTails tails;
+    __shared__ unsigned long long starts_s[CHAIN_CHUNKS];
     __shared__ int hist_s[3][TSP_HIST_BINS], max_s[3];
-    const int first = blockIdx.x * NB, tid = threadIdx.x;
-    for (int i = tid; i < NB + 8; i += 128)
-    {
-        const int b = first + i;
-        if (i < NB) { cls_s[i] = b < nb8 ? cls_of[b] : 2; tiles_s[i] = b < nb8 ? tiles_of[b] : 0; }
-        rp_s[i] = min(max(rowptr[b < nb8 ? b * 8 : rowA], 0), nnz);
-    }
-    for (int i = tid; i < 3 * TSP_HIST_BINS; i += 128) (&hist_s[0][0])[i] = 0;
+    const int tid = threadIdx.x, b = blockIdx.x * CHAIN_NB + tid, c = b / CHAIN_L, pos = b % CHAIN_L, len = min(CHAIN_L, nb8 - c * CHAIN_L);
+    for (int i = tid; i < 3 * TSP_HIST_BINS; i += CHAIN_NB) (&hist_s[0][0])[i] = 0;
     if (tid < 3) max_s[tid] = 0;
-    __syncthreads();
-    const int c = blockIdx.x * EMIT_CHUNKS + tid;
-    if (tid < EMIT_CHUNKS && c < nchunk)
+    const int k = b < nb8 ? cls_of[b] : 2, tl = b < nb8 ? tiles_of[b] : 0;
+    int en = 0;
+    if (b < nb8)
     {
-        int at[CHAIN_N];
+        const int e = b + step_of(k);
+        en = min(max(rowptr[e < nb8 ? e * 8 : rowA], 0), nnz) - min(max(rowptr[b * 8], 0), nnz);
+    }
+    cls_s[tid] = (unsigned char)k;
+    tails.build(pos, len, k, tl, en);   // ends with a barrier
+    if (pos == 0 && c < nchunk)
+    {
+        unsigned long long mask = 0;
+        for (int p = entry[c]; p < len; p += step_of(cls_s[tid + p])) mask |= 1ull << p;
+        starts_s[tid / CHAIN_L] = mask;
+    }
+    __syncthreads();
+    if (c < nchunk)
+    {
+        const int en0 = entry[c];
+        int at[CHAIN_N], tail[CHAIN_N];
 #pragma unroll
-        for (int q = 0; q < CHAIN_N; q++) at[q] = base[c * CHAIN_N + q];
-        int pos = c * CHAIN_L + entry[c], sq = at[0] + at[1] + at[2];
-        const int end = min((c + 1) * CHAIN_L, nb8);
-        while (pos < end)
+        for (int q = 0; q < CHAIN_N; q++) at[q] = 0;
+        if (en0 < len) tails.counts((tid & ~(CHAIN_L - 1)) + en0, at);
+#pragma unroll
+        for (int q = 0; q < CHAIN_N; q++) at[q] += base[c * CHAIN_N + q];   // behind the chunk
+        if (c == nchunk - 1 && pos == 0)
+#pragma unroll
+            for (int q = 0; q < 3; q++) { out.tile_ptr[q][at[q]] = at[3 + q]; out.nnz_ptr[q][at[q]] = at[6 + q]; }
+        if (pos < len && (starts_s[tid / CHAIN_L] >> pos & 1))
         {
-            const int k = cls_s[pos - first], step = step_of(k), tl = tiles_s[pos - first], en = rp_s[pos - first + step] - rp_s[pos - first];
+            tails.counts(tid, tail);
+#pragma unroll
+            for (int q = 0; q < CHAIN_N; q++) at[q] -= tail[q];             // at this panel
 #pragma unroll
             for (int q = 0; q < 3; q++)
                 if (q == k)
                 {
-                    out.tile_ptr[q][at[q]] = at[3 + q]; out.nnz_ptr[q][at[q]] = at[6 + q]; out.panel_row[q][at[q]] = pos * 8;
-                    if (seq.blk) { seq.blk[sq] = pos; seq.cls[sq] = (unsigned char)q; seq.idx[sq] = at[q]; seq.tiles[sq] = tl; }
-                    at[q]++; at[3 + q] += tl; at[6 + q] += en;
+                    out.tile_ptr[q][at[q]] = at[3 + q]; out.nnz_ptr[q][at[q]] = at[6 + q]; out.panel_row[q][at[q]] = b * 8;
+                    if (seq.blk)
+                    {
+                        const int sq = at[0] + at[1] + at[2];
+                        seq.blk[sq] = b; seq.cls[sq] = (unsigned char)q; seq.idx[sq] = at[q]; seq.tiles[sq] = tl;
+                    }
                 }
-            const int len = min(max(tl, 0), TSP_HIST_BINS - 1);
-            atomicAdd(&hist_s[k][len], 1);
+            atomicAdd(&hist_s[k][min(max(tl, 0), TSP_HIST_BINS - 1)], 1);
             atomicMax(&max_s[k], tl);
-            sq++;
-            pos += step;
-            if (pos >= nb8) st->last_cls = k;
+            if (b + step_of(k) >= nb8) st->last_cls = k;
         }
-        if (c == nchunk - 1)
-#pragma unroll
-            for (int q = 0; q < 3; q++) { out.tile_ptr[q][at[q]] = at[3 + q]; out.nnz_ptr[q][at[q]] = at[6 + q]; }
     }
     __syncthreads();
-    for (int i = tid; i < 3 * TSP_HIST_BINS; i += 128) { const int v = (&hist_s[0][0])[i]; if (v) atomicAdd(&(&st->hist[0][0])[i], v); }
+    for (int i = tid; i < 3 * TSP_HIST_BINS; i += CHAIN_NB) { const int v = (&hist_s[0][0])[i]; if (v) atomicAdd(&(&st->hist[0][0])[i], v); }
     if (tid < 3 && max_s[tid]) atomicMax(&st->max_len[tid], max_s[tid]);
 }
 
@@ -1647,10 +1703,10 @@ int tsp_convert_impl(tsp_handle *h, int rowA, int colA, long long nnz64, const i
             TSP_CUDA(cudaGetLastError());
         }
         mark("step 2 window counts");
-        k_chain_local<<<(nchunk + LOCAL_CHUNKS - 1) / LOCAL_CHUNKS, LOCAL_CHUNKS * 8, 0, st>>>(nb8, nchunk, rowA, nnz, prec, gamma, delta, fixed, reach, d_rowptr, ulen,
-                                                                                              fresh, cls_of, tiles_of, exit_off, counts);
+        k_chain_local<<<(nchunk + CHAIN_CHUNKS - 1) / CHAIN_CHUNKS, CHAIN_NB, 0, st>>>(nb8, nchunk, rowA, nnz, prec, gamma, delta, fixed, reach, d_rowptr, ulen,
+                                                                                      fresh, cls_of, tiles_of, exit_off, counts);
         k_chain_compose<<<1, 1024, 0, st>>>(nchunk, exit_off, counts, entry, base, d_stats);
-        k_chain_emit<<<(nchunk + EMIT_CHUNKS - 1) / EMIT_CHUNKS, 128, 0, st>>>(nb8, nchunk, rowA, nnz, cls_of, tiles_of, entry, base, d_rowptr, all, seq, d_stats);
+        k_chain_emit<<<(nchunk + CHAIN_CHUNKS - 1) / CHAIN_CHUNKS, CHAIN_NB, 0, st>>>(nb8, nchunk, rowA, nnz, cls_of, tiles_of, entry, base, d_rowptr, all, seq, d_stats);
         TSP_CUDA(cudaGetLastError());
         TSP_CUDA(cudaMemcpyAsync(pin, d_stats, sizeof(ConvStats), cudaMemcpyDeviceToHost, st));
         TSP_CUDA(cudaStreamSynchronize(st));
