@@ -1,5 +1,6 @@
 """GPU parity of the conversion where its kernels change method: blocks of exactly / one more than the entries a warp or a
-CTA sorts, lists longer than one slice of columns, more columns than one bitmap pass holds, repeated entries in short and
+CTA sorts, lists longer than one slice of columns, as many columns as the small
+bitmap holds and one more, more than one pass of the large one holds, repeated entries in short and
 long panels, a short last panel.  Bit-exact against the CPU checker, so there is no tolerance."""
 import numpy as np
 import pytest
@@ -34,7 +35,7 @@ def blocks_csr(sizes, cols, last_rows, repeats, seed):
 
 
 @pytest.mark.parametrize("prec", [0, 1])
-@pytest.mark.parametrize("cols,repeats", [(40000, False), (40000, True), ((1 << 20) + 5, False), (300, True)])
+@pytest.mark.parametrize("cols,repeats", [(40000, False), (40000, True), (1 << 18, False), ((1 << 18) + 1, True), ((1 << 20) + 5, False), (300, True)])
 def test_conversion_at_the_edges_of_its_methods(prec, cols, repeats):
     from tilespmm_b200 import api
     m = api.TileMatrix(prec)

@@ -39,6 +39,7 @@ namespace
 constexpr int CHAIN_L = 64;         // 8-row blocks per chunk of the chain resolution
 constexpr int SMALL_N = 512;        // entries a warp sorts in registers / builds tiles of in shared memory
 constexpr int MID_N = 4096;         // entries a CTA of 256 threads sorts in shared memory
+constexpr int MID_WORDS = 8192;     // words of the bitmap it uses instead when all columns fit
 constexpr int SLICE_COLS = 4096;    // distinct columns of one slice of a long panel
 constexpr int CHUNK_N = 4096;       // entries one CTA places into the records of a 64-row panel
 
@@ -225,40 +226,44 @@ __device__ __forceinline__ int cta_list(CtaTemp &temp, unsigned *last, int n, in
     return cta_sort_unique<16>(temp.t16, last, n, bits, load, emit);
 }
 
-// The same for any n by a CTA of 1024 threads with a bitmap of `words` (a multiple of 1024) shared 32-bit words: one pass
-// over the keys per words*32 columns.  A bitmap of all columns costs its own size, which for n > 4096 is less than sorting.
-template <typename Load, typename Emit>
-__device__ __forceinline__ int cta_bitmap_unique(unsigned *bm, int words, int *s_warp /* [33] */, int n, int colA, Load load, Emit emit)
+// The same for any n by a CTA of T threads with a bitmap of `words` (a multiple of 1024) shared 32-bit words: one pass
+// over the keys per words*32 columns.  A bitmap of all columns costs its own size (clear, count, read back), which is less
+// than sorting for n > 4096, and for n > 512 while the columns fit MID_WORDS.
+template <int T, typename Load, typename Emit>
+__device__ __forceinline__ int cta_bitmap_unique(unsigned *bm, int words, int *s_warp /* [T/32 + 1] */, int n, int colA, Load load, Emit emit)
 {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, per_warp = words / 32;
+    constexpr int W = T / 32;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, per_warp = words / W;
     int done = 0;
     for (long long lo = 0; lo < colA; lo += (long long)words * 32)
     {
-        for (int i = tid; i < words / 4; i += 1024) reinterpret_cast<uint4 *>(bm)[i] = make_uint4(0u, 0u, 0u, 0u);
+        for (int i = tid; i < words / 4; i += T) reinterpret_cast<uint4 *>(bm)[i] = make_uint4(0u, 0u, 0u, 0u);
         __syncthreads();
         const unsigned span = (unsigned)min((long long)words * 32, (long long)colA - lo), first = (unsigned)lo;
 #pragma unroll 4
-        for (int e = tid; e < n; e += 1024)
+        for (int e = tid; e < n; e += T)
         {
             const unsigned c = (unsigned)load(e) - first;
             if (c < span) atomicOr(&bm[c >> 5], 1u << (c & 31));
         }
         __syncthreads();
         int sum = 0;
+#pragma unroll 4
         for (int i = lane; i < per_warp; i += 32) sum += __popc(bm[warp * per_warp + i]);
         for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
         if (lane == 0) s_warp[warp] = sum;
         __syncthreads();
         if (warp == 0)
         {
-            const int v = s_warp[lane];
+            const int v = lane < W ? s_warp[lane] : 0;
             int incl = v;
             for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += y; }
-            s_warp[lane] = incl - v;
-            if (lane == 31) s_warp[32] = incl;
+            if (lane < W) s_warp[lane] = incl - v;
+            if (lane == 31) s_warp[W] = incl;
         }
         __syncthreads();
         int run = done + s_warp[warp];
+#pragma unroll 2
         for (int i = lane; i < per_warp; i += 32)
         {
             unsigned w = bm[warp * per_warp + i];
@@ -270,10 +275,31 @@ __device__ __forceinline__ int cta_bitmap_unique(unsigned *bm, int words, int *s
             while (w) { emit(pos++, (int)(first + (unsigned)(warp * per_warp + i) * 32u + (unsigned)__ffs(w) - 1u)); w &= w - 1; }
             run += __shfl_sync(0xffffffffu, incl, 31);
         }
-        done += s_warp[32];
+        done += s_warp[W];
         __syncthreads();
     }
     return done;
+}
+
+// up to MID_N keys by a CTA of 256 threads
+template <bool BITMAP>
+struct MidTemp
+{
+    CtaTemp sort;
+    unsigned last[256];
+};
+template <>
+struct MidTemp<true>
+{
+    __align__(16) unsigned bm[MID_WORDS];
+    int s_warp[9];
+};
+template <typename Load, typename Emit>
+__device__ __forceinline__ int mid_list(MidTemp<false> &t, int n, int bits, int, int, Load load, Emit emit) { return cta_list(t.sort, t.last, n, bits, load, emit); }
+template <typename Load, typename Emit>
+__device__ __forceinline__ int mid_list(MidTemp<true> &t, int n, int, int words, int colA, Load load, Emit emit)
+{
+    return cta_bitmap_unique<256>(t.bm, words, t.s_warp, n, colA, load, emit);
 }
 
 // ---- step 1: lists of the 8-row blocks, and the consistency check of the CSR
@@ -320,11 +346,12 @@ __global__ void __launch_bounds__(256) k_block_lists(int nb8, int rowA, int colA
     if (wrong) atomicExch(&st->bad, 1);
 }
 
-__global__ void __launch_bounds__(256) k_block_lists_mid(int rowA, int colA, int nnz, int bits, const int *__restrict__ rowptr, const int *__restrict__ colidx,
+// BITMAP: all columns fit MID_WORDS words and a bitmap replaces the radix sort (R-MAT scale 18, 2^18 columns: 81 -> 62 us)
+template <bool BITMAP>
+__global__ void __launch_bounds__(256) k_block_lists_mid(int rowA, int colA, int nnz, int bits, int words, const int *__restrict__ rowptr, const int *__restrict__ colidx,
                                                          int *__restrict__ ucols, int *__restrict__ ulen, const int *__restrict__ mid, ConvStats *st)
 {
-    __shared__ CtaTemp temp;
-    __shared__ unsigned last[256];
+    __shared__ MidTemp<BITMAP> temp;
     bool wrong = false;
     const int count = st->n_mid[0];
     for (int i = blockIdx.x; i < count; i += gridDim.x)
@@ -332,7 +359,7 @@ __global__ void __launch_bounds__(256) k_block_lists_mid(int rowA, int colA, int
         const int b = mid[i];
         int begin, n;
         block_range(b, rowA, nnz, rowptr, begin, n);
-        const int len = cta_list(temp, last, n, bits, [&](int e) { const int c = colidx[begin + e]; wrong |= c < 0 || c >= colA; return c; },
+        const int len = mid_list(temp, n, bits, words, colA, [&](int e) { const int c = colidx[begin + e]; wrong |= c < 0 || c >= colA; return c; },
                                  [&](int pos, int c) { ucols[begin + pos] = c; });
         if (threadIdx.x == 0) ulen[b] = len;
     }
@@ -351,7 +378,7 @@ __global__ void __launch_bounds__(1024) k_block_lists_big(int rowA, int colA, in
         const int b = big[i];
         int begin, n;
         block_range(b, rowA, nnz, rowptr, begin, n);
-        const int len = cta_bitmap_unique(bm, words, s_warp, n, colA, [&](int e) { const int c = colidx[begin + e]; wrong |= c < 0 || c >= colA; return c; },
+        const int len = cta_bitmap_unique<1024>(bm, words, s_warp, n, colA, [&](int e) { const int c = colidx[begin + e]; wrong |= c < 0 || c >= colA; return c; },
                                           [&](int pos, int c) { ucols[begin + pos] = c; });
         if (threadIdx.x == 0) ulen[b] = len;
     }
@@ -915,11 +942,11 @@ __global__ void __launch_bounds__(256) k_panel_lists(int nb8, int rowA, int prec
     }
 }
 
-__global__ void __launch_bounds__(256) k_panel_lists_mid(int nb8, int precision, int bits, const int *__restrict__ rowptr, const int *__restrict__ ucols,
+template <bool BITMAP>
+__global__ void __launch_bounds__(256) k_panel_lists_mid(int nb8, int colA, int precision, int bits, int words, const int *__restrict__ rowptr, const int *__restrict__ ucols,
                                                          const int *__restrict__ ulen, ClassView v64, ClassView v16, const int *__restrict__ mid, const ConvStats *st)
 {
-    __shared__ CtaTemp temp;
-    __shared__ unsigned last_s[256];
+    __shared__ MidTemp<BITMAP> temp;
     __shared__ Segments sg;
     const int count = st->n_mid[1];
     for (int w = blockIdx.x; w < count; w += gridDim.x)
@@ -930,7 +957,7 @@ __global__ void __launch_bounds__(256) k_panel_lists_mid(int nb8, int precision,
         if (threadIdx.x < 32) load_segments(sg, v.panel_row[p], v.cls, nb8, rowptr, ulen, threadIdx.x);
         __syncthreads();
         int *dst = v.tile_colidx + (size_t)t0 * bn;
-        const int d = cta_list(temp, last_s, sg.pre[8], bits, [&](int e) { return ucols[sg.find(e)]; }, [&](int pos, int c) { dst[pos] = c; });
+        const int d = mid_list(temp, sg.pre[8], bits, words, colA, [&](int e) { return ucols[sg.find(e)]; }, [&](int pos, int c) { dst[pos] = c; });
         const int last = dst[d - 1];
         for (int q = d + threadIdx.x; q < nt * bn; q += 256) dst[q] = last;
         __syncthreads();
@@ -952,7 +979,7 @@ __global__ void __launch_bounds__(1024) k_panel_lists_big(int nb8, int colA, int
         if (threadIdx.x < 32) load_segments(sg, v.panel_row[p], v.cls, nb8, rowptr, ulen, threadIdx.x);
         __syncthreads();
         int *dst = v.tile_colidx + (size_t)t0 * bn;
-        const int d = cta_bitmap_unique(bm, words, s_warp, sg.pre[8], colA, [&](int e) { return ucols[sg.find(e)]; }, [&](int pos, int c) { dst[pos] = c; });
+        const int d = cta_bitmap_unique<1024>(bm, words, s_warp, sg.pre[8], colA, [&](int e) { return ucols[sg.find(e)]; }, [&](int pos, int c) { dst[pos] = c; });
         const int last = dst[d - 1];
         for (int q = d + threadIdx.x; q < nt * bn; q += 1024) dst[q] = last;
         __syncthreads();
@@ -1691,7 +1718,8 @@ int tsp_convert_impl(tsp_handle *h, int rowA, int colA, long long nnz64, const i
     {
         TspRange range("tsp convert: partition (steps 1-3)");
         k_block_lists<<<capped((nb8 + 16 + 7) / 8, 148 * 64), T, 0, st>>>(nb8, rowA, colA, nnz, d_rowptr, d_colidx, ucols, ulen, mid, big, d_stats);
-        if (nnz > SMALL_N) k_block_lists_mid<<<capped(nnz / SMALL_N, 148 * 5), T, 0, st>>>(rowA, colA, nnz, bits, d_rowptr, d_colidx, ucols, ulen, mid, d_stats);
+        if (nnz > SMALL_N)
+            (words <= MID_WORDS ? k_block_lists_mid<true> : k_block_lists_mid<false>)<<<capped(nnz / SMALL_N, 148 * 6), T, 0, st>>>(rowA, colA, nnz, bits, words, d_rowptr, d_colidx, ucols, ulen, mid, d_stats);
         if (nnz > MID_N) k_block_lists_big<<<capped(nnz / MID_N, 148), 1024, words * 4, st>>>(rowA, colA, nnz, words, d_rowptr, d_colidx, ucols, ulen, big, d_stats);
         TSP_CUDA(cudaGetLastError());
         TSP_TRY(upload_values());   // the values go up on a side stream while the partition kernels run
@@ -1814,7 +1842,8 @@ int tsp_convert_impl(tsp_handle *h, int rowA, int colA, long long nnz64, const i
         const long long keys = h->cls[0].nnz + (long16 ? h->cls[1].nnz : 0);
         k_panel_lists<<<capped(((long long)h->cls[0].tilem + v16.tilem + 7) / 8, 148 * 32), T, 0, st>>>(nb8, rowA, prec, d_rowptr, ucols, ulen, view[0], v16, chunks, chunk_cap,
                                                                                                        mid, big, d_stats);
-        if (keys > SMALL_N) k_panel_lists_mid<<<capped(keys / SMALL_N, 148 * 5), T, 0, st>>>(nb8, prec, bits, d_rowptr, ucols, ulen, view[0], v16, mid, d_stats);
+        if (keys > SMALL_N)
+            (words <= MID_WORDS ? k_panel_lists_mid<true> : k_panel_lists_mid<false>)<<<capped(keys / SMALL_N, 148 * 6), T, 0, st>>>(nb8, colA, prec, bits, words, d_rowptr, ucols, ulen, view[0], v16, mid, d_stats);
         if (keys > MID_N) k_panel_lists_big<<<capped(keys / MID_N, 148), 1024, words * 4, st>>>(nb8, colA, prec, words, d_rowptr, ucols, ulen, view[0], v16, big, d_stats);
         TSP_CUDA(cudaGetLastError());
     }
