@@ -41,6 +41,10 @@ constexpr int SMALL_N = 512;        // entries a warp sorts in registers / build
 constexpr int MID_N = 4096;         // entries a CTA of 256 threads sorts in shared memory
 constexpr int MID_WORDS = 8192;     // words of the bitmap it uses instead when all columns fit
 constexpr int SLICE_COLS = 4096;    // distinct columns of one slice of a long panel
+constexpr int SLICE_T = 256;        // threads per slice (512: 4 - 10 % slower on R-MAT scale 18)
+// Entries a thread of the tile kernels has in hand at a time: one entry is a chain of a global load, 9 - 12 dependent
+// shared-memory loads and a store.  R-MAT scale 18, one entry -> four: short panels 118 -> 74 us, slices 170 -> 108 us.
+constexpr int FILL_U = 4;
 constexpr int CHUNK_N = 4096;       // entries one CTA places into the records of a 64-row panel
 
 // What the host reads back in one copy, and the counters of the device-side work lists.
@@ -1020,6 +1024,23 @@ __device__ __forceinline__ void add_in_csr_order(V *vals, unsigned long long pos
 }
 
 
+// number of elements of the ascending list a[0..n) below each of U keys; the U searches run side by side, so that a step
+// costs one shared-memory latency and not U
+template <int U>
+__device__ __forceinline__ void lower_bounds(const int *a, int n, const int (&key)[U], int (&pos)[U])
+{
+#pragma unroll
+    for (int u = 0; u < U; u++) pos[u] = 0;
+    for (int s = n > 0 ? 1 << (31 - __clz(n)) : 0; s > 0; s >>= 1)
+    {
+        int at[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) at[u] = a[min(pos[u] + s, n) - 1];
+#pragma unroll
+        for (int u = 0; u < U; u++) if (pos[u] + s <= n && at[u] < key[u]) pos[u] += s;
+    }
+}
+
 // the row of a panel that entry j belongs to: largest r with rp[r] <= j (BM rows, a power of two)
 template <int BM>
 __device__ __forceinline__ int row_of(const int *rp, int j)
@@ -1084,24 +1105,45 @@ __global__ void __launch_bounds__(128) k_fill_small(int nb8, int rowA, const int
         const int cols = nt * BN;
         for (int i = lane; i < nt * (int)(BM * BN * sizeof(V) / 16); i += 32) reinterpret_cast<uint4 *>(w.image)[i] = make_uint4(0u, 0u, 0u, 0u);
         for (int i = lane; i < (cols * BM + 31) / 32; i += 32) w.seen[i] = 0u;
-        for (int i = lane; i < nt; i += 32) w.tn[i] = 0;
         __syncwarp();
         const int last = w.list[d - 1];
         for (int i = d + lane; i < cols; i += 32) w.list[i] = last;   // src/csr2tile.h:117-132
         __syncwarp();
         for (int i = lane; i < cols; i += 32) v.tile_colidx[(size_t)t0 * BN + i] = w.list[i];
-        bool twice = false;
-        for (int e = lane; e < n; e += 32)
+        // FILL_U entries a lane at a time: loads, searches and stores of one do not wait for those of another.  Entries per
+        // tile are counted from the bits afterwards; fewer bits than entries means that one came twice.
+        for (int e0 = lane; e0 < n; e0 += 32 * FILL_U)
         {
-            const int j = begin + e, r = row_of<BM>(w.rp, j), rank = lower_bound_dev(w.list, d, colidx[j]), t = rank / BN;
-            const unsigned bit = (unsigned)(rank * BM + r), m = 1u << (bit & 31);
-            twice |= (atomicOr(&w.seen[bit >> 5], m) & m) != 0u;
-            atomicAdd(&w.tn[t], 1);
-            w.image[t * BM * BN + tsp_upstream_index(PREC, CLS, r, rank % BN)] = val[j];
+            int c[FILL_U], rank[FILL_U];
+            V x[FILL_U];
+#pragma unroll
+            for (int u = 0; u < FILL_U; u++) { const int j = begin + min(e0 + 32 * u, n - 1); c[u] = colidx[j]; x[u] = val[j]; }
+            lower_bounds<FILL_U>(w.list, d, c, rank);
+#pragma unroll
+            for (int u = 0; u < FILL_U; u++)
+            {
+                if (e0 + 32 * u >= n) break;
+                const int r = row_of<BM>(w.rp, begin + e0 + 32 * u);
+                const unsigned bit = (unsigned)(rank[u] * BM + r);
+                atomicOr(&w.seen[bit >> 5], 1u << (bit & 31));
+                w.image[rank[u] / BN * BM * BN + tsp_upstream_index(PREC, CLS, r, rank[u] % BN)] = x[u];
+            }
         }
-        if (__any_sync(0xffffffffu, twice))   // repeated entries: once more, row by row, adding in CSR order
+        __syncwarp();
+        int bits = 0;
+        for (int t = lane; t < nt; t += 32)
+        {
+            int cnt = 0;
+#pragma unroll
+            for (int q = 0; q < BM * BN / 32; q++) cnt += __popc(w.seen[t * (BM * BN / 32) + q]);
+            w.tn[t] = cnt;
+            bits += cnt;
+        }
+        for (int o = 16; o > 0; o >>= 1) bits += __shfl_xor_sync(0xffffffffu, bits, o);
+        if (bits != n)   // repeated entries: once more, row by row, adding in CSR order
         {
             __syncwarp();
+            for (int i = lane; i < nt; i += 32) w.tn[i] = 0;
             for (int i = lane; i < nt * (int)(BM * BN * sizeof(V) / 16); i += 32) reinterpret_cast<uint4 *>(w.image)[i] = make_uint4(0u, 0u, 0u, 0u);
             __syncwarp();
             for (int r = 0; r < BM; r++)
@@ -1116,6 +1158,7 @@ __global__ void __launch_bounds__(128) k_fill_small(int nb8, int rowA, const int
                         const int rank = lower_bound_dev(w.list, d, colidx[j]);
                         pos = (unsigned long long)(rank / BN * BM * BN + tsp_upstream_index(PREC, CLS, r, rank % BN));
                         x = val[j];
+                        atomicAdd(&w.tn[rank / BN], 1);
                     }
                     add_in_csr_order<V>(w.image, pos, x, on, lane);
                 }
@@ -1154,11 +1197,11 @@ __device__ __forceinline__ void write_tile_nnz(const int *tn, int nt, int before
 
 // Slices of long 16- and 8-row panels, a CTA each: it reads all entries of the panel and keeps those of its columns.
 template <typename V, int CLS>
-__global__ void __launch_bounds__(256) k_fill_slices(int rowA, const int *__restrict__ rowptr, const int *__restrict__ colidx, const V *__restrict__ val,
+__global__ void __launch_bounds__(SLICE_T) k_fill_slices(int rowA, const int *__restrict__ rowptr, const int *__restrict__ colidx, const V *__restrict__ val,
                                                      const int *__restrict__ ucols, const int *__restrict__ ulen, ClassView v, V *__restrict__ tiles, const ConvStats *st)
 {
     constexpr int PREC = sizeof(V) == 4 ? 1 : 0, BM = CLS == 1 ? 16 : 8, BN = PREC ? 8 : 16, PER = SLICE_COLS / BN;
-    __shared__ int list[SLICE_COLS], tn[PER], rp[BM + 1], s_before, s_twice;
+    __shared__ int list[SLICE_COLS], tn[PER], rp[BM + 1], s_before, s_more;
     __shared__ unsigned seen[SLICE_COLS * BM / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, count = min(st->n_items[CLS], v.item_cap), nnz0 = v.nnz_ptr[0];
     for (int w = blockIdx.x; w < count; w += gridDim.x)
@@ -1167,45 +1210,77 @@ __global__ void __launch_bounds__(256) k_fill_slices(int rowA, const int *__rest
         const int p = v.items[w].x, s = v.items[w].y, row0 = v.panel_row[p];
         const int t0 = v.tile_ptr[p] + s * PER, nt = min(v.tile_ptr[p + 1] - t0, PER), cols = nt * BN;
         if (tid <= BM) rp[tid] = rowptr[row0 + min(tid, rowA - row0)];
-        if (tid == 0) { s_before = 0; s_twice = 0; }
-        for (int i = tid; i < nt; i += 256) tn[i] = 0;
-        for (int i = tid; i < (cols * BM + 31) / 32; i += 256) seen[i] = 0u;
+        if (tid == 0) { s_before = 0; s_more = 0; }
+        for (int i = tid; i < (cols * BM + 31) / 32; i += SLICE_T) seen[i] = 0u;
         uint4 *z = reinterpret_cast<uint4 *>(tiles + (size_t)t0 * BM * BN);
         const int z16 = nt * (int)(BM * BN * sizeof(V) / 16);
-        for (int i = tid; i < z16; i += 256) z[i] = make_uint4(0u, 0u, 0u, 0u);
+        for (int i = tid; i < z16; i += SLICE_T) z[i] = make_uint4(0u, 0u, 0u, 0u);
         int *ci = v.tile_colidx + (size_t)t0 * BN;
         if (CLS == 2)
         {
             const int d = ulen[row0 / 8] - s * SLICE_COLS;
             const int *src = ucols + rowptr[row0] + s * SLICE_COLS;
-            for (int i = tid; i < cols; i += 256) { const int c = src[min(i, d - 1)]; list[i] = c; ci[i] = c; }   // padded with the last column
+            for (int i = tid; i < cols; i += SLICE_T) { const int c = src[min(i, d - 1)]; list[i] = c; ci[i] = c; }   // padded with the last column
         }
-        else for (int i = tid; i < cols; i += 256) list[i] = ci[i];
+        else for (int i = tid; i < cols; i += SLICE_T) list[i] = ci[i];
         __syncthreads();
         const int lo = list[0], hi = list[cols - 1];
-        int before = 0;
-        bool twice = false;
-#pragma unroll 2
-        for (int j = rp[0] + tid; j < rp[BM]; j += 256)
+        int before = 0, hits = 0;
+        const unsigned n = (unsigned)(rp[BM] - rp[0]);   // unsigned: the last steps may pass 2^31
+        for (unsigned e0 = tid; e0 < n; e0 += SLICE_T * FILL_U)
         {
-            const int c = colidx[j];
-            before += c < lo;
-            if (c < lo || c > hi) continue;
-            const int r = row_of<BM>(rp, j), rank = lower_bound_dev(list, cols, c), t = rank / BN;
-            const unsigned bit = (unsigned)(rank * BM + r), m = 1u << (bit & 31);
-            twice |= (atomicOr(&seen[bit >> 5], m) & m) != 0u;
-            atomicAdd(&tn[t], 1);
-            tiles[(size_t)(t0 + t) * (BM * BN) + tsp_upstream_index(PREC, CLS, r, rank % BN)] = val[j];
+            int c[FILL_U], rank[FILL_U];
+            bool in[FILL_U], any = false;
+#pragma unroll
+            for (int u = 0; u < FILL_U; u++) c[u] = colidx[rp[0] + (int)min(e0 + SLICE_T * u, n - 1)];
+#pragma unroll
+            for (int u = 0; u < FILL_U; u++)
+            {
+                const bool on = e0 + SLICE_T * u < n;
+                before += on && c[u] < lo;
+                in[u] = on && c[u] >= lo && c[u] <= hi;
+                hits += in[u];
+                any |= in[u];
+            }
+            if (!any) continue;
+            V x[FILL_U];
+#pragma unroll
+            for (int u = 0; u < FILL_U; u++) if (in[u]) x[u] = val[rp[0] + (int)(e0 + SLICE_T * u)];
+            lower_bounds<FILL_U>(list, cols, c, rank);
+#pragma unroll
+            for (int u = 0; u < FILL_U; u++)
+            {
+                if (!in[u]) continue;
+                const int r = row_of<BM>(rp, rp[0] + (int)(e0 + SLICE_T * u)), t = rank[u] / BN;
+                const unsigned bit = (unsigned)(rank[u] * BM + r);
+                atomicOr(&seen[bit >> 5], 1u << (bit & 31));
+                tiles[(size_t)(t0 + t) * (BM * BN) + tsp_upstream_index(PREC, CLS, r, rank[u] % BN)] = x[u];
+            }
         }
         for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+        for (int o = 16; o > 0; o >>= 1) hits += __shfl_xor_sync(0xffffffffu, hits, o);
         if (lane == 0 && before) atomicAdd(&s_before, before);
-        if (twice) s_twice = 1;
+        if (lane == 0 && hits) atomicAdd(&s_more, hits);
         __syncthreads();
-        if (s_twice)
+        // entries per tile from the bits; s_more becomes the number of entries that fell on a bit already set
+        int bits = 0;
+        for (int t = tid; t < nt; t += SLICE_T)
         {
-            for (int i = tid; i < z16; i += 256) z[i] = make_uint4(0u, 0u, 0u, 0u);
+            int cnt = 0;
+#pragma unroll
+            for (int q = 0; q < BM * BN / 32; q++) cnt += __popc(seen[t * (BM * BN / 32) + q]);
+            tn[t] = cnt;
+            bits += cnt;
+        }
+        for (int o = 16; o > 0; o >>= 1) bits += __shfl_xor_sync(0xffffffffu, bits, o);
+        if (lane == 0 && bits) atomicSub(&s_more, bits);
+        __syncthreads();
+        if (s_more)
+        {
+            for (int i = tid; i < nt; i += SLICE_T) tn[i] = 0;
+            for (int i = tid; i < z16; i += SLICE_T) z[i] = make_uint4(0u, 0u, 0u, 0u);
             __syncthreads();
-            for (int r = warp; r < BM; r += 8)
+            for (int r = warp; r < BM; r += SLICE_T / 32)
                 for (int base = rp[r]; base < rp[r + 1]; base += 32)
                 {
                     const int j = base + lane, c = j < rp[r + 1] ? colidx[j] : -1;
@@ -1217,10 +1292,12 @@ __global__ void __launch_bounds__(256) k_fill_slices(int rowA, const int *__rest
                         const int rank = lower_bound_dev(list, cols, c);
                         pos = (unsigned long long)(t0 + rank / BN) * (BM * BN) + (unsigned long long)tsp_upstream_index(PREC, CLS, r, rank % BN);
                         x = val[j];
+                        atomicAdd(&tn[rank / BN], 1);
                     }
                     add_in_csr_order<V>(tiles, pos, x, on, lane);
                 }
         }
+        __syncthreads();
         write_tile_nnz(tn, nt, v.nnz_ptr[p] - nnz0 + s_before, v.tile_nnz + t0);
     }
 }
@@ -1265,16 +1342,32 @@ __global__ void __launch_bounds__(256) k_masks64(int rowA, const int *__restrict
         const int lo = m.list[0], hi = m.list[cols - 1];
         int before = 0;
         bool twice = false;
-#pragma unroll 2
-        for (int j = m.rp[0] + tid; j < m.rp[64]; j += 256)
+        const unsigned n = (unsigned)(m.rp[64] - m.rp[0]);
+        for (unsigned e0 = tid; e0 < n; e0 += 256 * FILL_U)
         {
-            const int c = colidx[j];
-            before += c < lo;
-            if (c < lo || c > hi) continue;
-            const int r = row_of<64>(m.rp, j), rank = lower_bound_dev(m.list, cols, c), t = rank / BN;
-            const unsigned bit = (unsigned)((t * 64 + r) * BN + rank % BN), b = 1u << (bit & 31);
-            twice |= (atomicOr(&m.masks[bit >> 5], b) & b) != 0u;
-            atomicAdd(&m.tn[t], 1);
+            int c[FILL_U], rank[FILL_U];
+            bool in[FILL_U], any = false;
+#pragma unroll
+            for (int u = 0; u < FILL_U; u++) c[u] = colidx[m.rp[0] + (int)min(e0 + 256 * u, n - 1)];
+#pragma unroll
+            for (int u = 0; u < FILL_U; u++)
+            {
+                const bool on = e0 + 256 * u < n;
+                before += on && c[u] < lo;
+                in[u] = on && c[u] >= lo && c[u] <= hi;
+                any |= in[u];
+            }
+            if (!any) continue;
+            lower_bounds<FILL_U>(m.list, cols, c, rank);
+#pragma unroll
+            for (int u = 0; u < FILL_U; u++)
+            {
+                if (!in[u]) continue;
+                const int r = row_of<64>(m.rp, m.rp[0] + (int)(e0 + 256 * u)), t = rank[u] / BN;
+                const unsigned bit = (unsigned)((t * 64 + r) * BN + rank[u] % BN), b = 1u << (bit & 31);
+                twice |= (atomicOr(&m.masks[bit >> 5], b) & b) != 0u;
+                atomicAdd(&m.tn[t], 1);
+            }
         }
         for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
         if (lane == 0 && before) atomicAdd(&m.before, before);
@@ -1471,7 +1564,7 @@ int fill_class(tsp_handle *h, int nb8, const int *rowptr, const int *colidx, con
     k_fill_small<V, CLS><<<capped((v.tilem + F::WARPS - 1) / F::WARPS, 148 * 32), 32 * F::WARPS, F::SMEM, st>>>(nb8, h->rowA, rowptr, colidx, val, ucols, ulen, v, tiles, d_stats);
     // a panel is long when it has more than SMALL_N entries or more than small_cols() - BN columns, hence as many entries
     if (entries > small_cols(F::PREC, CLS) - F::BN)
-        k_fill_slices<V, CLS><<<capped(v.item_cap, 148 * 8), 256, 0, st>>>(h->rowA, rowptr, colidx, val, ucols, ulen, v, tiles, d_stats);
+        k_fill_slices<V, CLS><<<capped(v.item_cap, 148 * (2048 / SLICE_T)), SLICE_T, 0, st>>>(h->rowA, rowptr, colidx, val, ucols, ulen, v, tiles, d_stats);
     TSP_CUDA(cudaGetLastError());
     return TSP_OK;
 }
