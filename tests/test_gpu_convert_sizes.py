@@ -103,3 +103,39 @@ def test_schedule_at_the_edge_of_the_one_block_builder(tasks):
         torch.cuda.synchronize()
         np.testing.assert_array_equal(C[: shape[0], 0].cpu().numpy(), np.diff(rp).astype(np.float32))
     m.close()
+
+
+@pytest.mark.parametrize("panels", [2049, 2303, 2304, 2305])
+def test_schedule_by_counting_sort(panels):
+    """More panels than the one-block builder takes: slices of equal and of rest length, several panels per CTA edge, lengths
+    beyond the 256 keys of the sort; the task arrays against plain Python, and every tile walked exactly once."""
+    import torch
+    from tilespmm_b200 import api
+    rng = np.random.default_rng(panels)
+    tiles = rng.integers(0, 6, size=panels)
+    tiles[rng.choice(panels, size=12, replace=False)] = (7, 8, 9, 31, 33, 64, 255, 256, 257, 300, 600, 601)
+    per_row = np.zeros(8 * panels, np.int64)
+    per_row[::8] = tiles * 16                                             # FP16 tiles hold 16 columns
+    rp = np.concatenate([[0], np.cumsum(per_row)]).astype(np.int32)
+    ci = np.concatenate([np.arange(n) for n in per_row]).astype(np.int32)
+    shape = (8 * panels, 16 * 601)
+    m = api.TileMatrix(0).convert_host(shape, rp, ci, np.ones(ci.size, np.float32), 5.0, 3.0)
+    B = torch.ones((shape[1], 32), dtype=torch.float16, device="cuda")
+    C = torch.full((m.c_rows(), 32), 7.0, dtype=torch.float32, device="cuda")
+    for TH in (1, 8, 64, 255, 256, 300, 1000):
+        rows, start = m.schedule(2, TH)
+        want_rows, want_start, t = [], [], 0
+        for p, n in enumerate(tiles.tolist()):
+            parts = 1 if n <= TH else -(-n // TH)
+            each = -(-n // parts)
+            for s in range(parts):
+                want_rows.append(8 * p | (0x80000000 if parts > 1 else 0))
+                want_start.append(t + s * each)
+            t += n
+        np.testing.assert_array_equal(rows, np.array(want_rows, np.uint32))
+        np.testing.assert_array_equal(start, np.array(want_start + [t], np.int32))
+        C.fill_(7.0)
+        m.spmm(B, C, 32)
+        torch.cuda.synchronize()
+        np.testing.assert_array_equal(C[: shape[0], 3].cpu().numpy(), per_row.astype(np.float32))
+    m.close()

@@ -1589,12 +1589,12 @@ void tsp_free_tiles(tsp_handle *h, bool release)
     {
         TspClass &c = h->cls[k];
         TspClass fresh;
-        if (release) { cudaFree(c.d_task_row); cudaFree(c.d_task_start); cudaFree(c.d_split_row); cudaFree(c.d_task_count); cudaFree(c.d_task_pack); }
+        if (release) { cudaFree(c.d_task_row); cudaFree(c.d_task_start); cudaFree(c.d_split_row); cudaFree(c.d_task_pack); }
         else
         {
             // the schedule arrays and their capacities survive: cudaFree/cudaMalloc per conversion cost more than the conversion kernels
             fresh.d_task_row = c.d_task_row; fresh.d_task_start = c.d_task_start; fresh.d_split_row = c.d_split_row;
-            fresh.d_task_count = c.d_task_count; fresh.d_task_pack = c.d_task_pack;
+            fresh.d_task_pack = c.d_task_pack;
             fresh.cap_tasks = c.cap_tasks; fresh.cap_panels = c.cap_panels;
         }
         c = fresh;

@@ -33,34 +33,11 @@ __global__ void k_task_counts(int tilem, const int *__restrict__ tile_ptr, int T
     counts[p] = len <= TH ? 1 : (len + TH - 1) / TH;  // src/csr2tile.h:392-396
 }
 
-__global__ void k_task_fill(int tilem, const int *__restrict__ tile_ptr, const int *__restrict__ panel_row, int TH,
-                            const int *__restrict__ task_base, unsigned int *__restrict__ task_row, int *__restrict__ task_start,
-                            int *__restrict__ split_row, int *__restrict__ split_count)
-{
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= tilem) return;
-    const int t0 = tile_ptr[p], len = tile_ptr[p + 1] - t0, b = task_base[p], row = panel_row[p];
-    if (p == 0) task_start[0] = t0;
-    if (len <= TH)
-    {
-        task_row[b] = (unsigned int)row;
-        task_start[b + 1] = t0 + len;
-        return;
-    }
-    const int parts = (len + TH - 1) / TH, each = (len + parts - 1) / parts;  // src/csr2tile.h:421-422
-    for (int s = 0; s < parts; s++)
-    {
-        task_row[b + s] = (unsigned int)row | 0x80000000u;
-        task_start[b + s + 1] = s == parts - 1 ? t0 + len : t0 + (s + 1) * each;
-    }
-    split_row[atomicAdd(split_count, 1)] = row;
-}
-
 // One class in one CTA, for at most SCHED_PANELS panels and SCHED_TASKS tasks: task counts, their prefix sum, the tasks,
 // and (pack != nullptr) the same tasks longest first.  Small matrices pay for launches, not for work: this is one launch
 // where the general path below takes seven.
 constexpr int SCHED_T = 512, SCHED_PANELS = 2048, SCHED_TASKS = 2048;
-__global__ void __launch_bounds__(SCHED_T) k_schedule_small(int tilem, const int *__restrict__ tile_ptr, const int *__restrict__ panel_row, int TH, int sorted,
+__global__ void __launch_bounds__(SCHED_T) k_schedule_small(int tilem, const int *__restrict__ tile_ptr, const int *__restrict__ panel_row, int TH, int top, int key_bits /* 0: panel order */,
                                                          unsigned int *__restrict__ task_row, int *__restrict__ task_start, int *__restrict__ split_row, uint4 *__restrict__ pack)
 {
     using Scan = cub::BlockScan<int, SCHED_T>;
@@ -107,9 +84,9 @@ __global__ void __launch_bounds__(SCHED_T) k_schedule_small(int tilem, const int
     for (int i = 0; i < SCHED_TASKS / SCHED_T; i++)
     {
         const int t = tid * (SCHED_TASKS / SCHED_T) + i;
-        key[i] = t < ntasks ? (0xffffu - (unsigned)min(starts[t + 1] - starts[t], 0xffff)) << 16 | (unsigned)t : 0xffffffffu;
+        key[i] = t < ntasks ? (unsigned)min(max(top - (starts[t + 1] - starts[t]), 0), 0xfffe) << 16 | (unsigned)t : 0xffffffffu;
     }
-    if (sorted) Sort(temp.sort).Sort(key, 16, 32);
+    if (key_bits) Sort(temp.sort).Sort(key, 16, 16 + key_bits);   // a length takes 1 - 8 bits as a rule, four to a pass
 #pragma unroll
     for (int i = 0; i < SCHED_TASKS / SCHED_T; i++)
     {
@@ -118,23 +95,131 @@ __global__ void __launch_bounds__(SCHED_T) k_schedule_small(int tilem, const int
     }
 }
 
-// sort key of a task: longer tasks get smaller keys (`top` bounds the lengths; the keys need bits_of(top) bits)
-__global__ void k_task_keys(int ntasks, unsigned top, const int *__restrict__ task_start, unsigned int *__restrict__ keys, int *__restrict__ ids)
+// In-place exclusive scan of a[0..n) by ONE block of exactly 1024 threads (all 32 warp_sum slots are written every
+// pass); n <= about a million ints: a few passes.
+constexpr int SCAN_THREADS = 1024;
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_one_block(int *a, int n)
 {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= ntasks) return;
-    const unsigned len = (unsigned)(task_start[t + 1] - task_start[t]);
-    keys[t] = top - (len > top ? top : len);
-    ids[t] = t;
+    __shared__ int warp_sum[32];
+    __shared__ int carry;
+    if (threadIdx.x == 0) carry = 0;
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int base = 0; base < n; base += blockDim.x)
+    {
+        const int i = base + threadIdx.x;
+        const int v = i < n ? a[i] : 0;
+        int x = v;
+        for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, x, o); if (lane >= o) x += y; }
+        if (lane == 31) warp_sum[warp] = x;
+        __syncthreads();
+        if (warp == 0)
+        {
+            int w = warp_sum[lane];
+            for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, w, o); if (lane >= o) w += y; }
+            warp_sum[lane] = w;
+        }
+        __syncthreads();
+        const int before = carry + (warp ? warp_sum[warp - 1] : 0) + x - v;
+        if (i < n) a[i] = before;
+        __syncthreads();
+        if (threadIdx.x == blockDim.x - 1) carry = before + v;
+        __syncthreads();
+    }
 }
 
-__global__ void k_task_pack(int ntasks, const int *__restrict__ order, const unsigned int *__restrict__ task_row,
-                            const int *__restrict__ task_start, uint4 *__restrict__ pack)
+// The general path: a stable counting sort of the tasks by length, panel by panel.  All slices of a panel but the last have
+// the same length, so a panel is two (length, count) pairs and nothing is ever sorted task by task.
+//   k_sched_count  a CTA per SCHED_BLOCK panels: its tasks per key, [key][CTA], and behind the keys its tasks altogether
+//   one prefix sum over that table
+//   k_sched_place  the same CTAs: the panels' tasks in panel order and, at their sorted places, in `pack`
+// These and the scan replace ten launches (counts, scan, fill, keys, three-kernel radix sort, pack),
+// R-MAT scale 18, 40,000 tasks: 41 -> 23 us and seven launches fewer.
+constexpr int SCHED_BLOCK = 256, SCHED_KEYS = 256;
+constexpr int SCHED_ONE_BLOCK_SCAN = 8192;   // table cells up to which one CTA scans (8 passes, one launch instead of two)
+
+// key of a task of `len` tiles: longer tasks first; a key stands for 1 << shift lengths
+__device__ __forceinline__ int sched_key(int len, int top, int shift) { return (top - len) >> shift; }
+
+// a panel's slices: `parts - 1` of `each` tiles and one of `last` (src/csr2tile.h:392-396, 421-422)
+struct PanelParts
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= ntasks) return;
-    const int t = order ? order[i] : i;
-    pack[i] = make_uint4(task_row[t], (unsigned int)task_start[t], (unsigned int)task_start[t + 1], 0u);
+    int t0, parts, each, last;
+    __device__ __forceinline__ PanelParts(const int *__restrict__ tile_ptr, int p, int TH)
+    {
+        t0 = tile_ptr[p];
+        const int len = tile_ptr[p + 1] - t0;
+        parts = len <= TH ? 1 : (len + TH - 1) / TH;
+        each = (len + parts - 1) / parts;
+        last = len - (parts - 1) * each;
+    }
+};
+
+__global__ void __launch_bounds__(SCHED_BLOCK) k_sched_count(int tilem, const int *__restrict__ tile_ptr, int TH, int top, int shift, int keys, int *__restrict__ table,
+                                                             int *__restrict__ split_count)
+{
+    __shared__ int hist[SCHED_KEYS + 1];
+    const int p = blockIdx.x * SCHED_BLOCK + threadIdx.x;
+    for (int i = threadIdx.x; i <= keys; i += SCHED_BLOCK) hist[i] = 0;
+    if (p == 0) *split_count = 0;
+    __syncthreads();
+    if (p < tilem)
+    {
+        const PanelParts q(tile_ptr, p, TH);
+        atomicAdd(&hist[sched_key(q.last, top, shift)], 1);
+        if (q.parts > 1) atomicAdd(&hist[sched_key(q.each, top, shift)], q.parts - 1);
+        atomicAdd(&hist[keys], q.parts);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i <= keys; i += SCHED_BLOCK) table[(size_t)i * gridDim.x + blockIdx.x] = hist[i];
+}
+
+__global__ void __launch_bounds__(SCHED_BLOCK) k_sched_place(int tilem, const int *__restrict__ tile_ptr, const int *__restrict__ panel_row, int TH, int top, int shift,
+                                                             int keys, int ntasks, const int *__restrict__ table, unsigned int *__restrict__ task_row,
+                                                             int *__restrict__ task_start, int *__restrict__ split_row, int *__restrict__ split_count, uint4 *__restrict__ pack)
+{
+    __shared__ int4 s_panel[SCHED_BLOCK];   // key and number of the equal slices, key of the last one, all slices
+    const int tid = threadIdx.x, p = blockIdx.x * SCHED_BLOCK + tid, mates = min(SCHED_BLOCK, tilem - (int)blockIdx.x * SCHED_BLOCK);
+    const PanelParts q(tile_ptr, min(p, tilem - 1), TH);
+    const int key = q.parts > 1 ? sched_key(q.each, top, shift) : -1, key_last = sched_key(q.last, top, shift);
+    s_panel[tid] = make_int4(key, q.parts - 1, key_last, q.parts);
+    __syncthreads();
+    const bool on = p < tilem;
+    int base = 0, at = 0, at_last = key == key_last ? q.parts - 1 : 0;   // tasks, equal keys, equal keys of the last slice before this one in the CTA
+    for (int j = 0; j < mates; j++)
+    {
+        const int4 o = s_panel[j];
+        if (j >= tid) break;
+        base += o.w;
+        at += (o.x == key ? o.y : 0) + (o.z == key ? 1 : 0);
+        at_last += (o.x == key_last ? o.y : 0) + (o.z == key_last ? 1 : 0);
+    }
+    base += table[(size_t)keys * gridDim.x + blockIdx.x] - ntasks;   // the table's last row is scanned behind all tasks of the keys
+    if (key >= 0) at += table[(size_t)key * gridDim.x + blockIdx.x];
+    at_last += table[(size_t)key_last * gridDim.x + blockIdx.x];
+    const int row = panel_row[min(p, tilem - 1)];
+    const unsigned word = (unsigned)row | (q.parts > 1 ? 0x80000000u : 0u);
+    auto write = [&](int i, int to, unsigned w, int start, int tiles) {
+        task_row[i] = w;
+        task_start[i] = start;
+        if (pack) pack[to] = make_uint4(w, (unsigned)start, (unsigned)(start + tiles), 0u);
+    };
+    if (on)
+    {
+        write(base + q.parts - 1, at_last, word, q.t0 + (q.parts - 1) * q.each, q.last);
+        if (p == tilem - 1) task_start[base + q.parts] = q.t0 + (q.parts - 1) * q.each + q.last;
+        if (q.parts > 1) split_row[atomicAdd(split_count, 1)] = row;
+    }
+    // the equal slices of a panel by all lanes of its warp: a hub's panel has hundreds
+    __syncwarp();
+    for (unsigned todo = __ballot_sync(0xffffffffu, on && q.parts > 1); todo; todo &= todo - 1)
+    {
+        const int l = __ffs(todo) - 1;
+        const int n = __shfl_sync(0xffffffffu, q.parts - 1, l), b = __shfl_sync(0xffffffffu, base, l), to = __shfl_sync(0xffffffffu, at, l);
+        const int t0 = __shfl_sync(0xffffffffu, q.t0, l), each = __shfl_sync(0xffffffffu, q.each, l);
+        const unsigned w = __shfl_sync(0xffffffffu, word, l);
+        for (int s = tid & 31; s < n; s += 32) write(b + s, to + s, w, t0 + s * each, each);
+    }
 }
 
 // The 16/8-row kernels run four tasks per CTA, one per warp, and a CTA holds its SM resources until its longest
@@ -195,12 +280,11 @@ int tsp_schedule_on(tsp_handle *h, int cls, int TH, cudaStream_t s)
         if (parts > 1) nsplit += hist[len];
     }
     if (ntasks > 0x7fffffffLL) { tsp_set_error("schedule: %lld tasks", ntasks); return TSP_EINVAL; }
-    if (!c.d_task_count || c.tilem > c.cap_panels)
+    if (!c.d_split_row || c.tilem > c.cap_panels)
     {
-        cudaFree(c.d_task_count); cudaFree(c.d_split_row);
-        c.d_task_count = nullptr; c.d_split_row = nullptr; c.cap_panels = 0;
-        TSP_CUDA(cudaMalloc((void **)&c.d_task_count, ((size_t)c.tilem + 2) * 4));
-        TSP_CUDA(cudaMalloc((void **)&c.d_split_row, ((size_t)c.tilem + 1) * 4));
+        cudaFree(c.d_split_row);
+        c.d_split_row = nullptr; c.cap_panels = 0;
+        TSP_CUDA(cudaMalloc((void **)&c.d_split_row, ((size_t)c.tilem + 1) * 4));   // the last word counts them
         c.cap_panels = c.tilem;
     }
     if (ntasks > c.cap_tasks)
@@ -214,44 +298,40 @@ int tsp_schedule_on(tsp_handle *h, int cls, int TH, cudaStream_t s)
         if (cls != 0) TSP_CUDA(cudaMalloc((void **)&c.d_task_pack, (size_t)cap * sizeof(uint4)));
         c.cap_tasks = cap;
     }
-    const int T = 256, n = (int)ntasks;
+    const int n = (int)ntasks;
     const bool sorted = tasks_sorted();
+    // task lengths are at most TH and at most the longest panel
+    const int top = (int)(hist.size() - 1 < (size_t)TH ? hist.size() - 1 : (size_t)TH);
     if (c.tilem <= SCHED_PANELS && n <= SCHED_TASKS)
     {
-        k_schedule_small<<<1, SCHED_T, 0, s>>>(c.tilem, c.d_tile_ptr, c.d_panel_row, TH, sorted ? 1 : 0, c.d_task_row, c.d_task_start, c.d_split_row,
+        int key_bits = 1;   // the largest key, all ones, stands for no task
+        while (key_bits < 16 && ((top + 1) >> key_bits)) key_bits++;
+        k_schedule_small<<<1, SCHED_T, 0, s>>>(c.tilem, c.d_tile_ptr, c.d_panel_row, TH, top, sorted ? key_bits : 0, c.d_task_row, c.d_task_start, c.d_split_row,
                                            cls != 0 ? c.d_task_pack : nullptr);
         TSP_CUDA(cudaGetLastError());
         c.ntasks = n; c.nsplit = (int)nsplit;
         return TSP_OK;
     }
-    // task lengths are at most TH and at most the longest panel: one pass of the sort for lengths below 256
-    unsigned top = (unsigned)(hist.size() - 1 < (size_t)TH ? hist.size() - 1 : (size_t)TH);
-    if (top > 0xffffu) top = 0xffffu;
-    int key_bits = 1;
-    while (key_bits < 16 && (top >> key_bits)) key_bits++;
-    size_t scan_bytes = 0, sort_bytes = 0;
-    unsigned *keys = nullptr, *keys_out = nullptr;
-    int *ids = nullptr, *ids_out = nullptr;
-    TSP_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, c.d_task_count, c.d_task_count, c.tilem + 1, s));
+    int shift = 0;
+    while ((top >> shift) >= SCHED_KEYS) shift++;
+    // without sorting all tasks share key 0 and keep panel order
     const bool sorting = cls != 0 && sorted;
-    if (sorting) TSP_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, keys, keys_out, ids, ids_out, n, 0, key_bits, s));
-    size_t cub_bytes = (scan_bytes > sort_bytes ? scan_bytes : sort_bytes) + 256;
-    cub_bytes = (cub_bytes + 255) & ~(size_t)255;
+    if (!sorting) shift = 31;
+    const int keys = (top >> shift) + 1, blocks = (c.tilem + SCHED_BLOCK - 1) / SCHED_BLOCK, cells = (keys + 1) * blocks;
+    const bool one_block = cells <= SCHED_ONE_BLOCK_SCAN;
+    size_t scan_bytes = 0;
+    int *table = nullptr;
+    if (!one_block) TSP_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, table, table, cells, s));
+    scan_bytes = (scan_bytes + 255) & ~(size_t)255;
     unsigned char *scratch;
-    TSP_TRY(sched_scratch(h, cub_bytes + (sorting ? (size_t)n * 16 : 0), &scratch));
-    k_task_counts<<<(c.tilem + 1 + T - 1) / T, T, 0, s>>>(c.tilem, c.d_tile_ptr, TH, c.d_task_count);
-    TSP_CUDA(cub::DeviceScan::ExclusiveSum(scratch, scan_bytes, c.d_task_count, c.d_task_count, c.tilem + 1, s));
-    int *d_split_count = c.d_task_count + c.tilem + 1;
-    TSP_CUDA(cudaMemsetAsync(d_split_count, 0, 4, s));
-    k_task_fill<<<(c.tilem + T - 1) / T, T, 0, s>>>(c.tilem, c.d_tile_ptr, c.d_panel_row, TH, c.d_task_count, c.d_task_row, c.d_task_start,
-                                                   c.d_split_row, d_split_count);
-    if (sorting)
-    {
-        keys = (unsigned *)(scratch + cub_bytes); keys_out = keys + n; ids = (int *)(keys + 2 * (size_t)n); ids_out = ids + n;
-        k_task_keys<<<(n + T - 1) / T, T, 0, s>>>(n, top, c.d_task_start, keys, ids);
-        TSP_CUDA(cub::DeviceRadixSort::SortPairs(scratch, sort_bytes, keys, keys_out, ids, ids_out, n, 0, key_bits, s));
-    }
-    if (cls != 0) k_task_pack<<<(n + T - 1) / T, T, 0, s>>>(n, sorting ? ids_out : nullptr, c.d_task_row, c.d_task_start, c.d_task_pack);
+    TSP_TRY(sched_scratch(h, scan_bytes + (size_t)cells * 4, &scratch));
+    table = reinterpret_cast<int *>(scratch + scan_bytes);
+    int *split_count = c.d_split_row + c.cap_panels;
+    k_sched_count<<<blocks, SCHED_BLOCK, 0, s>>>(c.tilem, c.d_tile_ptr, TH, top, shift, keys, table, split_count);
+    if (one_block) k_scan_one_block<<<1, SCAN_THREADS, 0, s>>>(table, cells);
+    else TSP_CUDA(cub::DeviceScan::ExclusiveSum(scratch, scan_bytes, table, table, cells, s));
+    k_sched_place<<<blocks, SCHED_BLOCK, 0, s>>>(c.tilem, c.d_tile_ptr, c.d_panel_row, TH, top, shift, keys, n, table, c.d_task_row, c.d_task_start,
+                                              c.d_split_row, split_count, cls != 0 ? c.d_task_pack : nullptr);
     TSP_CUDA(cudaGetLastError());
     c.ntasks = n; c.nsplit = (int)nsplit;
     return TSP_OK;
@@ -391,40 +471,7 @@ static __device__ __align__(256) int g_noalloc_scratch[TSP_NOALLOC_MAX_PANELS + 
 namespace
 {
 
-// In-place exclusive scan of a[0..n) by ONE block of exactly 1024 threads (all 32 warp_sum slots are written every
-// pass); n <= about a million ints: a few passes.
-constexpr int SCAN_THREADS = 1024;
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_one_block(int *a, int n)
-{
-    __shared__ int warp_sum[32];
-    __shared__ int carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int base = 0; base < n; base += blockDim.x)
-    {
-        const int i = base + threadIdx.x;
-        const int v = i < n ? a[i] : 0;
-        int x = v;
-        for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, x, o); if (lane >= o) x += y; }
-        if (lane == 31) warp_sum[warp] = x;
-        __syncthreads();
-        if (warp == 0)
-        {
-            int w = warp_sum[lane];
-            for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, w, o); if (lane >= o) w += y; }
-            warp_sum[lane] = w;
-        }
-        __syncthreads();
-        const int before = carry + (warp ? warp_sum[warp - 1] : 0) + x - v;
-        if (i < n) a[i] = before;
-        __syncthreads();
-        if (threadIdx.x == blockDim.x - 1) carry = before + v;
-        __syncthreads();
-    }
-}
-
-// Same output as k_task_fill, but never writes past the caller's capacity.
+// The tasks in panel order from the scanned counts; never writes past the caller's capacity.
 __global__ void k_task_fill_bounded(int tilem, const int *__restrict__ tile_ptr, const int *__restrict__ panel_row, int TH,
                                     const int *__restrict__ task_base, long long capacity, unsigned int *__restrict__ task_row,
                                     int *__restrict__ task_start, int *__restrict__ split_row, int *__restrict__ split_count)

@@ -154,7 +154,7 @@ struct TspClass
     int TH = 0, ntasks = 0, nsplit = 0;
     long long cap_tasks = 0, cap_panels = 0;   // capacities of the task arrays / the per-panel arrays (kept across conversions)
     unsigned int *d_task_row = nullptr;
-    int *d_task_start = nullptr, *d_split_row = nullptr, *d_task_count = nullptr;
+    int *d_task_start = nullptr, *d_split_row = nullptr;
     // the same tasks as {row word, first tile, end tile, 0}, longest first (what the 16/8-row kernels walk)
     uint4 *d_task_pack = nullptr;
 };
