@@ -230,7 +230,7 @@ __device__ __forceinline__ int cta_list(CtaTemp &temp, unsigned *last, int n, in
     return cta_sort_unique<16>(temp.t16, last, n, bits, load, emit);
 }
 
-// The same for any n by a CTA of T threads with a bitmap of `words` (a multiple of 1024) shared 32-bit words: one pass
+// The same for any n by a CTA of T threads with a bitmap of `words` (a multiple of 4096) shared 32-bit words: one pass
 // over the keys per words*32 columns.  A bitmap of all columns costs its own size (clear, count, read back), which is less
 // than sorting for n > 4096, and for n > 512 while the columns fit MID_WORDS.
 template <int T, typename Load, typename Emit>
@@ -251,9 +251,10 @@ __device__ __forceinline__ int cta_bitmap_unique(unsigned *bm, int words, int *s
             if (c < span) atomicOr(&bm[c >> 5], 1u << (c & 31));
         }
         __syncthreads();
+        const uint4 *mine = reinterpret_cast<const uint4 *>(bm) + warp * (per_warp / 4);
         int sum = 0;
 #pragma unroll 4
-        for (int i = lane; i < per_warp; i += 32) sum += __popc(bm[warp * per_warp + i]);
+        for (int i = lane; i < per_warp / 4; i += 32) { const uint4 w = mine[i]; sum += __popc(w.x) + __popc(w.y) + __popc(w.z) + __popc(w.w); }
         for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
         if (lane == 0) s_warp[warp] = sum;
         __syncthreads();
@@ -267,16 +268,17 @@ __device__ __forceinline__ int cta_bitmap_unique(unsigned *bm, int words, int *s
         }
         __syncthreads();
         int run = done + s_warp[warp];
-#pragma unroll 2
-        for (int i = lane; i < per_warp; i += 32)
+        for (int i = lane; i < per_warp / 4; i += 32)   // four words a lane: one prefix sum for 128 words
         {
-            unsigned w = bm[warp * per_warp + i];
-            const int c = __popc(w);
+            const uint4 w = mine[i];
+            const int c = __popc(w.x) + __popc(w.y) + __popc(w.z) + __popc(w.w);
             int incl = c;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += y; }
             int pos = run + incl - c;
-            while (w) { emit(pos++, (int)(first + (unsigned)(warp * per_warp + i) * 32u + (unsigned)__ffs(w) - 1u)); w &= w - 1; }
+            const unsigned col0 = first + (unsigned)(warp * per_warp + 4 * i) * 32u;
+            auto words_of = [&](unsigned x, unsigned at) { while (x) { emit(pos++, (int)(at + (unsigned)__ffs(x) - 1u)); x &= x - 1; } };
+            words_of(w.x, col0); words_of(w.y, col0 + 32u); words_of(w.z, col0 + 64u); words_of(w.w, col0 + 96u);
             run += __shfl_sync(0xffffffffu, incl, 31);
         }
         done += s_warp[W];
@@ -350,7 +352,7 @@ __global__ void __launch_bounds__(256) k_block_lists(int nb8, int rowA, int colA
     if (wrong) atomicExch(&st->bad, 1);
 }
 
-// BITMAP: all columns fit MID_WORDS words and a bitmap replaces the radix sort (R-MAT scale 18, 2^18 columns: 81 -> 62 us)
+// BITMAP: all columns fit MID_WORDS words and a bitmap replaces the radix sort (R-MAT scale 18, 2^18 columns: 81 -> 52 us)
 template <bool BITMAP>
 __global__ void __launch_bounds__(256) k_block_lists_mid(int rowA, int colA, int nnz, int bits, int words, const int *__restrict__ rowptr, const int *__restrict__ colidx,
                                                          int *__restrict__ ucols, int *__restrict__ ulen, const int *__restrict__ mid, ConvStats *st)
@@ -1524,7 +1526,7 @@ int bits_for(unsigned long long v)
 // shared words of the bitmap kernels: all columns when they fit 128 KB (2^20 columns), else several passes
 int bitmap_words(int colA)
 {
-    const long long w = ((long long)colA + 32767) / 32768 * 1024;
+    const long long w = ((long long)colA + 131071) / 131072 * 4096;   // every warp of a CTA reads whole uint4 rows
     return w > 32768 ? 32768 : (int)w;
 }
 
@@ -1813,7 +1815,7 @@ int tsp_convert_impl(tsp_handle *h, int rowA, int colA, long long nnz64, const i
         k_block_lists<<<capped((nb8 + 16 + 7) / 8, 148 * 64), T, 0, st>>>(nb8, rowA, colA, nnz, d_rowptr, d_colidx, ucols, ulen, mid, big, d_stats);
         if (nnz > SMALL_N)
             (words <= MID_WORDS ? k_block_lists_mid<true> : k_block_lists_mid<false>)<<<capped(nnz / SMALL_N, 148 * 6), T, 0, st>>>(rowA, colA, nnz, bits, words, d_rowptr, d_colidx, ucols, ulen, mid, d_stats);
-        if (nnz > MID_N) k_block_lists_big<<<capped(nnz / MID_N, 148), 1024, words * 4, st>>>(rowA, colA, nnz, words, d_rowptr, d_colidx, ucols, ulen, big, d_stats);
+        if (nnz > MID_N) k_block_lists_big<<<capped(nnz / MID_N, 148 * 2), 1024, words * 4, st>>>(rowA, colA, nnz, words, d_rowptr, d_colidx, ucols, ulen, big, d_stats);
         TSP_CUDA(cudaGetLastError());
         TSP_TRY(upload_values());   // the values go up on a side stream while the partition kernels run
         mark("step 1 block lists");
@@ -1937,7 +1939,7 @@ int tsp_convert_impl(tsp_handle *h, int rowA, int colA, long long nnz64, const i
                                                                                                        mid, big, d_stats);
         if (keys > SMALL_N)
             (words <= MID_WORDS ? k_panel_lists_mid<true> : k_panel_lists_mid<false>)<<<capped(keys / SMALL_N, 148 * 6), T, 0, st>>>(nb8, colA, prec, bits, words, d_rowptr, ucols, ulen, view[0], v16, mid, d_stats);
-        if (keys > MID_N) k_panel_lists_big<<<capped(keys / MID_N, 148), 1024, words * 4, st>>>(nb8, colA, prec, words, d_rowptr, ucols, ulen, view[0], v16, big, d_stats);
+        if (keys > MID_N) k_panel_lists_big<<<capped(keys / MID_N, 148 * 2), 1024, words * 4, st>>>(nb8, colA, prec, words, d_rowptr, ucols, ulen, view[0], v16, big, d_stats);
         TSP_CUDA(cudaGetLastError());
     }
     mark("step 5 panel lists");
