@@ -108,17 +108,19 @@ def test_schedule_at_the_edge_of_the_one_block_builder(tasks):
 @pytest.mark.parametrize("panels", [2049, 2303, 2304, 2305])
 def test_schedule_by_counting_sort(panels):
     """More panels than the one-block builder takes: slices of equal and of rest length, several panels per CTA edge, lengths
-    beyond the 256 keys of the sort; the task arrays against plain Python, and every tile walked exactly once."""
+    beyond the 256 keys of the sort, lengths from 1024 tiles on, which the conversion hands over one by one; the task arrays against plain Python, and every tile walked exactly once."""
     import torch
     from tilespmm_b200 import api
     rng = np.random.default_rng(panels)
     tiles = rng.integers(0, 6, size=panels)
-    tiles[rng.choice(panels, size=12, replace=False)] = (7, 8, 9, 31, 33, 64, 255, 256, 257, 300, 600, 601)
+    tiles[rng.choice(panels, size=14, replace=False)] = (7, 8, 9, 31, 33, 64, 255, 256, 257, 300, 1023, 1024, 1024, 1025)
+    if panels == 2305:
+        tiles[:257] = 1024                                                # more long panels than the conversion lists
     per_row = np.zeros(8 * panels, np.int64)
     per_row[::8] = tiles * 16                                             # FP16 tiles hold 16 columns
     rp = np.concatenate([[0], np.cumsum(per_row)]).astype(np.int32)
     ci = np.concatenate([np.arange(n) for n in per_row]).astype(np.int32)
-    shape = (8 * panels, 16 * 601)
+    shape = (8 * panels, 16 * 1025)
     m = api.TileMatrix(0).convert_host(shape, rp, ci, np.ones(ci.size, np.float32), 5.0, 3.0)
     B = torch.ones((shape[1], 32), dtype=torch.float16, device="cuda")
     C = torch.full((m.c_rows(), 32), 7.0, dtype=torch.float32, device="cuda")

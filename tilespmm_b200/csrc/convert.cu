@@ -11,7 +11,7 @@
 //      not hold (binary searches in their lists).  The distinct columns of a window are sums of eight such counts.
 //   3. the upstream decision (64 / 16 / 8 rows) for EVERY 8-aligned start, with the same float comparisons, then the
 //      greedy chain i <- i + step(i), resolved chunk-wise; the same pass carries tiles and entries per class, so the
-//      chain's last kernel writes tile_ptr and the histogram of panel lengths directly.
+//      chain's last kernel writes tile_ptr and the panels by length directly.
 //   4. ONE read-back of a few kilobytes; allocation.
 //   5. tall panels: sorted distinct columns from the lists of their blocks (the same three methods), written as
 //      tile_colidx.
@@ -29,6 +29,7 @@
 #include <stdlib.h>
 #include <sys/time.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "tsp_internal.cuh"
@@ -55,8 +56,9 @@ struct ConvStats
     int panels[3], tiles[3], nnz[3];
     int n_mid[2], n_big[2];         // blocks / panels left to the CTA-level list kernels
     int n_items[3], n_chunks;       // slices of long panels; chunks of entries of 64-row panels
-    int max_len[3];                 // longest panel in tiles
-    int hist[3][TSP_HIST_BINS];     // panels by number of tiles; the last bin stands for every longer one
+    int n_long[3];                  // panels of TSP_HIST_BINS and more tiles; cleared with all that follows
+    int hist[3][TSP_HIST_BINS];     // panels by number of tiles
+    int long_len[3][TSP_LONG_PANELS];   // tiles of the long ones, in any order
 };
 
 // Bump allocator over the handle's workspace chunks.  The first conversion sizes chunk 0 from nnz and rowA; what
@@ -716,6 +718,12 @@ struct SeqArrays
     unsigned char *cls;
 };
 
+__device__ __forceinline__ void note_long_panel(ConvStats *st, int k, int tiles)
+{
+    const int at = atomicAdd(&st->n_long[k], 1);
+    if (at < TSP_LONG_PANELS) st->long_len[k][at] = tiles;
+}
+
 // Writes the panels of every chunk.  One thread per chunk follows the chain from its true entry and marks the blocks that
 // start panels; then every block knows from the tails what lies between the entry and itself.
 __global__ void __launch_bounds__(CHAIN_NB)
@@ -725,10 +733,9 @@ k_chain_emit(int nb8, int nchunk, int rowA, int nnz, const unsigned char *__rest
     __shared__ unsigned char cls_s[CHAIN_NB];
     __shared__ ChainTails tails;
     __shared__ unsigned long long starts_s[CHAIN_CHUNKS];
-    __shared__ int hist_s[3][TSP_HIST_BINS], max_s[3];
+    __shared__ int hist_s[3][TSP_HIST_BINS];
     const int tid = threadIdx.x, b = blockIdx.x * CHAIN_NB + tid, c = b / CHAIN_L, pos = b % CHAIN_L, len = min(CHAIN_L, nb8 - c * CHAIN_L);
     for (int i = tid; i < 3 * TSP_HIST_BINS; i += CHAIN_NB) (&hist_s[0][0])[i] = 0;
-    if (tid < 3) max_s[tid] = 0;
     const int k = b < nb8 ? cls_of[b] : 2, tl = b < nb8 ? tiles_of[b] : 0;
     int en = 0;
     if (b < nb8)
@@ -773,14 +780,13 @@ k_chain_emit(int nb8, int nchunk, int rowA, int nnz, const unsigned char *__rest
                         seq.blk[sq] = b; seq.cls[sq] = (unsigned char)q; seq.idx[sq] = at[q]; seq.tiles[sq] = tl;
                     }
                 }
-            atomicAdd(&hist_s[k][min(max(tl, 0), TSP_HIST_BINS - 1)], 1);
-            atomicMax(&max_s[k], tl);
+            if (tl < TSP_HIST_BINS) atomicAdd(&hist_s[k][max(tl, 0)], 1);
+            else note_long_panel(st, k, tl);
             if (b + step_of(k) >= nb8) st->last_cls = k;
         }
     }
     __syncthreads();
     for (int i = tid; i < 3 * TSP_HIST_BINS; i += CHAIN_NB) { const int v = (&hist_s[0][0])[i]; if (v) atomicAdd(&(&st->hist[0][0])[i], v); }
-    if (tid < 3 && max_s[tid]) atomicMax(&st->max_len[tid], max_s[tid]);
 }
 
 // ---- shard selection on the device: a contiguous range of the panel sequence, balanced by tile bytes
@@ -858,8 +864,8 @@ __global__ void k_shard_stats(ClassArrays all, int3 p0, int3 p1, ConvStats *st)
         if (i == 0) { st->tiles[k] = all.tile_ptr[k][a + n] - all.tile_ptr[k][a]; st->nnz[k] = all.nnz_ptr[k][a + n] - all.nnz_ptr[k][a]; }
         if (i >= n) continue;
         const int len = all.tile_ptr[k][a + i + 1] - all.tile_ptr[k][a + i];
-        atomicAdd(&st->hist[k][min(len, TSP_HIST_BINS - 1)], 1);
-        atomicMax(&st->max_len[k], len);
+        if (len < TSP_HIST_BINS) atomicAdd(&st->hist[k][len], 1);
+        else note_long_panel(st, k, len);
     }
 }
 
@@ -1873,7 +1879,7 @@ int tsp_convert_impl(tsp_handle *h, int rowA, int colA, long long nnz64, const i
         if (cuts[1] < nseq || cuts[0] >= cuts[1]) short_cls = -1;
         int most = 0;
         for (int k = 0; k < 3; k++) if (p1[k] - p0[k] > most) most = p1[k] - p0[k];
-        TSP_CUDA(cudaMemsetAsync(d_stats->max_len, 0, sizeof(ConvStats) - offsetof(ConvStats, max_len), st));
+        TSP_CUDA(cudaMemsetAsync(d_stats->n_long, 0, sizeof(ConvStats) - offsetof(ConvStats, n_long), st));
         k_shard_stats<<<blocks_for(most, T), T, 0, st>>>(all, make_int3(p0[0], p0[1], p0[2]), make_int3(p1[0], p1[1], p1[2]), d_stats);
         TSP_CUDA(cudaGetLastError());
         TSP_CUDA(cudaMemcpyAsync(pin, d_stats, sizeof(ConvStats), cudaMemcpyDeviceToHost, st));
@@ -1892,8 +1898,17 @@ int tsp_convert_impl(tsp_handle *h, int rowA, int colA, long long nnz64, const i
             for (int q = 0; q < 3; q++) if (q != k) others += (long long)(p1[q] - p0[q]) * tsp_bm(q);
             c.rows = (int)((long long)(h->row_end - h->row_begin) - others);
         }
-        c.max_len = pin->max_len[k];
-        if (c.max_len < TSP_HIST_BINS - 1) c.len_hist.assign(pin->hist[k], pin->hist[k] + c.max_len + 1);
+        if (pin->n_long[k] <= TSP_LONG_PANELS)
+        {
+            for (int len = 0, left = c.tilem - pin->n_long[k]; len < TSP_HIST_BINS && left > 0; left -= pin->hist[k][len++])
+                if (pin->hist[k][len]) c.lengths.push_back({len, pin->hist[k][len]});
+            std::sort(pin->long_len[k], pin->long_len[k] + pin->n_long[k]);
+            for (int i = 0; i < pin->n_long[k]; i++)
+            {
+                if (c.lengths.empty() || c.lengths.back().first != pin->long_len[k][i]) c.lengths.push_back({pin->long_len[k][i], 0});
+                c.lengths.back().second++;
+            }
+        }
     }
 
     // ---- step 4: the tile arrays of all classes, one allocation

@@ -2,12 +2,13 @@
 //
 // Replaces upstream get_optimal_prefetch_th (src/csr2tile.h:437-642), tile_pretreatment (src/csr2tile.h:383-434)
 // and update_metadata (src/csr2tile.h:644-711).  The task arrays are built on the device from tile_ptr
-// (upstream: host loop + upload per tuning combination); the cost model runs on the host over the histogram
-// of tiles per panel, in float and in upstream's evaluation order, with the resource rows of THESE kernels.
+// (upstream: host loop + upload per tuning combination); the cost model runs on the host over the
+// panels' lengths in tiles, in float and in upstream's evaluation order, with the resource rows of THESE kernels.
 #include <cub/cub.cuh>
 #include <math.h>
 #include <stdlib.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "tsp_internal.cuh"
@@ -246,38 +247,47 @@ int sched_scratch(tsp_handle *h, size_t bytes, unsigned char **p)
     return TSP_OK;
 }
 
-// panels by number of tiles, from the conversion's histogram or from tile_ptr
-int length_histogram(const tsp_handle *h, int cls, std::vector<int> &hist)
+using Lengths = std::vector<std::pair<int, int>>;
+
+// {tiles, panels of that many tiles} of a class, ascending: the conversion's, or counted from tile_ptr
+int panel_lengths(const tsp_handle *h, int cls, Lengths &own, const Lengths *&out)
 {
     const TspClass &c = h->cls[cls];
-    if (!c.len_hist.empty()) { hist = c.len_hist; return TSP_OK; }
+    out = &c.lengths;
+    if (!c.lengths.empty()) return TSP_OK;
     TSP_TRY(tsp_fetch_panels(h, cls));
     const std::vector<int> &tp = c.h_tile_ptr;
-    int max_len = 0;
-    for (int p = 0; p < c.tilem; p++) max_len = tp[p + 1] - tp[p] > max_len ? tp[p + 1] - tp[p] : max_len;
-    hist.assign((size_t)max_len + 1, 0);
-    for (int p = 0; p < c.tilem; p++) hist[tp[p + 1] - tp[p]]++;
+    std::vector<int> all((size_t)c.tilem);
+    for (int p = 0; p < c.tilem; p++) all[p] = tp[p + 1] - tp[p];
+    std::sort(all.begin(), all.end());
+    for (int len : all)
+    {
+        if (own.empty() || own.back().first != len) own.push_back({len, 0});
+        own.back().second++;
+    }
+    out = &own;
     return TSP_OK;
 }
 
 }  // namespace
 
 // Enqueues the task arrays of class cls for threshold TH on `s`.  How many tasks and split panels there will be follows
-// from the histogram of panel lengths, so nothing is read back and the host does not wait.
+// from the panels' lengths, so nothing is read back and the host does not wait.
 int tsp_schedule_on(tsp_handle *h, int cls, int TH, cudaStream_t s)
 {
     TspRange range("tsp schedule");
     TspClass &c = h->cls[cls];
     c.TH = TH; c.ntasks = 0; c.nsplit = 0;
     if (c.tilem == 0) return TSP_OK;
-    std::vector<int> hist;
-    TSP_TRY(length_histogram(h, cls, hist));
+    Lengths own;
+    const Lengths *lengths;
+    TSP_TRY(panel_lengths(h, cls, own, lengths));
     long long ntasks = 0, nsplit = 0;
-    for (size_t len = 0; len < hist.size(); len++)
+    for (const auto &l : *lengths)
     {
-        const long long parts = (long long)len <= TH ? 1 : ((long long)len + TH - 1) / TH;
-        ntasks += parts * hist[len];
-        if (parts > 1) nsplit += hist[len];
+        const long long parts = l.first <= TH ? 1 : ((long long)l.first + TH - 1) / TH;
+        ntasks += parts * l.second;
+        if (parts > 1) nsplit += l.second;
     }
     if (ntasks > 0x7fffffffLL) { tsp_set_error("schedule: %lld tasks", ntasks); return TSP_EINVAL; }
     if (!c.d_split_row || c.tilem > c.cap_panels)
@@ -301,7 +311,7 @@ int tsp_schedule_on(tsp_handle *h, int cls, int TH, cudaStream_t s)
     const int n = (int)ntasks;
     const bool sorted = tasks_sorted();
     // task lengths are at most TH and at most the longest panel
-    const int top = (int)(hist.size() - 1 < (size_t)TH ? hist.size() - 1 : (size_t)TH);
+    const int top = std::min(lengths->back().first, TH);
     if (c.tilem <= SCHED_PANELS && n <= SCHED_TASKS)
     {
         int key_bits = 1;   // the largest key, all ones, stands for no task
@@ -393,14 +403,12 @@ int tsp_top4(const tsp_handle *h, int cls, int colB, int *top4)
     const float lambda_atom = tsp_atom_weight(is_tf32, cls, colB);
     const float atom_per_col = lambda_atom * (1.0f / 32.0f);
 
-    std::vector<int> hist;
-    TSP_TRY(length_histogram(h, cls, hist));
-    const int max_len = (int)hist.size() - 1;
+    Lengths own;
+    const Lengths *lengths;
+    TSP_TRY(panel_lengths(h, cls, own, lengths));
+    const int max_len = lengths->back().first;
     const long long total_len = c.tilenum;
     if (max_len <= 0) return TSP_OK;
-    hist[0] = 0;
-    std::vector<int> lens;
-    for (int len = 1; len <= max_len; len++) if (hist[len]) lens.push_back(len);
 
     const float avg_len = (float)total_len / c.tilem;
     float atom_pen = atom_per_col * (float)colB;
@@ -417,15 +425,25 @@ int tsp_top4(const tsp_handle *h, int cls, int colB, int *top4)
         long long atom_ops = 0, tasks = 0;
         int max_chunk = 0;
         float l2_penalty = 0.0f;
-        for (int len : lens)
+        // the lengths ascend, so the number of parts only grows; within one number of parts the longest panel has the largest slice
+        int parts = 1, longest = 0;
+        float share = 0.0f;   // 1 - 1 / parts
+        for (const auto &l : *lengths)
         {
-            const int cnt = hist[len];
-            const int parts = (len + TH - 1) / TH, each = (len + parts - 1) / parts;
+            const int len = l.first, cnt = l.second;
+            if (len == 0) continue;
+            if ((long long)len > (long long)parts * TH)
+            {
+                if (longest && (longest + parts - 1) / parts > max_chunk) max_chunk = (longest + parts - 1) / parts;
+                parts = (len + TH - 1) / TH;
+                share = 1.0f - (1.0f / (float)parts);
+            }
+            longest = len;
             atom_ops += (long long)(parts - 1) * cnt;
             tasks += (long long)parts * cnt;
-            if (each > max_chunk) max_chunk = each;
-            if (parts > 1) l2_penalty += (1.0f - (1.0f / (float)parts)) * cnt;
+            if (parts > 1) l2_penalty += share * cnt;
         }
+        if ((longest + parts - 1) / parts > max_chunk) max_chunk = (longest + parts - 1) / parts;
         if (tasks == prev_tasks) continue;
         prev_tasks = tasks;
         const long long blocks = (tasks * (colB / stripe) + R.tasks_per_block - 1) / R.tasks_per_block;

@@ -128,7 +128,8 @@ struct TspKernelResources  // what the platform probe records per (class, width)
     long long shared_bytes;
 };
 
-#define TSP_HIST_BINS 1024
+#define TSP_HIST_BINS 1024     // panels are counted by length below this many tiles, longer ones are listed one by one
+#define TSP_LONG_PANELS 256
 
 struct TspClass
 {
@@ -146,10 +147,9 @@ struct TspClass
     unsigned char *d_pack = nullptr;
     long long pack_bytes = 0;
     mutable std::vector<int> h_tile_ptr, h_panel_row;   // host copies, fetched on first use (tsp_fetch_panels)
-    // panels by number of tiles (index = tiles), what the threshold model and the schedule sizes are computed from; empty
-    // when a panel is too long for it (max_len >= TSP_HIST_BINS - 1) or after tsp_load: then h_tile_ptr serves
-    std::vector<int> len_hist;
-    int max_len = 0;
+    // {tiles, panels of that many tiles}, ascending: what the threshold model and the schedule sizes are computed from.
+    // Filled by the conversion; empty after tsp_load or with more than TSP_LONG_PANELS long panels: then h_tile_ptr serves
+    std::vector<std::pair<int, int>> lengths;
     // schedule for the current threshold
     int TH = 0, ntasks = 0, nsplit = 0;
     long long cap_tasks = 0, cap_panels = 0;   // capacities of the task arrays / the per-panel arrays (kept across conversions)
